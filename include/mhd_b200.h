@@ -363,7 +363,9 @@ int mhd_batch_tune_candidates(int which, int* out, int cap);
  * ng = 2).  The reverse pass
  * differentiates the time step and c_h through the CFL argmax cell, the psi
  * damping and every branch the forward took, recomputing the trajectory from
- * checkpoints kept every `checkpoint_every` steps (0: about sqrt(nsteps)).
+ * checkpoints kept every `checkpoint_every` steps (0: about sqrt(nsteps), or,
+ * where every step's two states fit an eighth of the free device memory, all of
+ * them, so that nothing is recomputed).
  * dtype MHD_F64 or MHD_F32 selects the precision of forward and adjoint. */
 typedef struct mhd_adjoint mhd_adjoint;
 int mhd_adjoint_create(int nx, int ny, int dtype, int limiter, double gamma, double cfl, double cr, int nsteps,

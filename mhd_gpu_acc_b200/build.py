@@ -3,6 +3,7 @@
 Per-file flags matter for numerics:
   step_f64.cu   --fmad=false      FP64 step, bit-exact with the reference CPU path
   step_f32.cu   --use_fast_math   FP32-bulk step
+  adj_f32.cu    --use_fast_math   FP32 adjoint sweeps
 Everything else uses the defaults.  The CUDA runtime is linked statically so the
 library only needs the driver at run time.
 
@@ -38,6 +39,8 @@ CU_SOURCES = {
     "ic_kernels.cu": ["--fmad=false"],
     "batch_api.cu": [],
     "adjoint.cu": [],
+    "adj_f64.cu": [],
+    "adj_f32.cu": ["--use_fast_math"],
 }
 CXX_SOURCES = {"cases.cpp": []}
 HEADERS = [f for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))] if os.path.isdir(CSRC) else []

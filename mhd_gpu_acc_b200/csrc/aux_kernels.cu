@@ -194,6 +194,7 @@ __global__ void clock_init_kernel(DevClock* c, const unsigned long long* max0) {
     c->status = CLK_OK;
     c->lowbeta_hits = 0u;
     c->flux_fallbacks = 0u;
+    c->log = nullptr;
 }
 
 unsigned grid_for(long long n, int threads) {

@@ -20,9 +20,12 @@ namespace mhd {
 
 constexpr int BX_WARPS = 4;  // warps per batched x-sweep CTA
 
+// The device table holds every instance twice, with P.parity 0 and then 1, so that
+// the kernels read an instance's parameters where they lie instead of copying
+// them per thread.
 struct BatchInst {
     DevGrid U, T;
-    StepParams P;  // physics, boundary types, t_end and clock of this instance
+    StepParams P;  // physics, boundary types, t_end, clock and step parity of this instance
     int x_segs, x_pad_;      // x-sweep segments per row
     int y_strips, y_bands;   // 32-column strips; bands of seg rows
     int y_units;             // ceil(strips * bands / YS_WARPS)
@@ -46,8 +49,7 @@ constexpr int bx_smem_bytes() { return BX_WARPS * XRing<PH>::kWarpBytes; }
 
 template <class PH>
 __global__ void __launch_bounds__(32 * BX_WARPS, PH::kXBlocks) batch_x_kernel(const BatchInst* __restrict__ inst,
-                                                              const int* __restrict__ first, int n, int parity,
-                                                              int rpw) {
+                                                              const int* __restrict__ first, int n, int rpw) {
     using V = typename Slot16<typename PH::Real>::V;
     extern __shared__ __align__(16) unsigned char bx_smem[];
     const int warp = threadIdx.x >> 5;
@@ -57,14 +59,13 @@ __global__ void __launch_bounds__(32 * BX_WARPS, PH::kXBlocks) batch_x_kernel(co
     for (int u = blockIdx.x; u < total; u += gridDim.x) {
         const int k = find_instance(first, n, u);
         const int local = u - __ldg(first + k);
-        StepParams P = inst[k].P;
-        P.parity = parity;
+        const StepParams& P = inst[k].P;
         double dt, ch, damp;
         if (!step_scalars(P, dt, ch, damp)) {
             if (local == 0 && threadIdx.x == 0) clock_flag_skip(P);
             continue;
         }
-        if (local == 0 && threadIdx.x == 0) P.clock->maxbits[parity ^ 1] = 0ull;
+        if (local == 0 && threadIdx.x == 0) P.clock->maxbits[P.parity ^ 1] = 0ull;
         const DevGrid& U = inst[k].U;
         const long long task = (long long)local * BX_WARPS + warp;
         if (task < (long long)inst[k].x_segs * U.ny) {  // whole warp
@@ -76,8 +77,7 @@ __global__ void __launch_bounds__(32 * BX_WARPS, PH::kXBlocks) batch_x_kernel(co
 
 template <class PH>
 __global__ void __launch_bounds__(32 * YS_WARPS, PH::kYBlocks) batch_y_kernel(const BatchInst* __restrict__ inst,
-                                                               const int* __restrict__ first, int n, int parity,
-                                                               int seg) {
+                                                               const int* __restrict__ first, int n, int seg) {
     using R = typename PH::Real;
     __shared__ __align__(16) R carry[PH::kYCarry ? YS_WARPS * YCarry<PH>::kSlots * 32 : 1];
     const int total = __ldg(first + n);
@@ -85,8 +85,7 @@ __global__ void __launch_bounds__(32 * YS_WARPS, PH::kYBlocks) batch_y_kernel(co
     for (int u = blockIdx.x; u < total; u += gridDim.x) {
         const int k = find_instance(first, n, u);
         const int local = u - __ldg(first + k);
-        StepParams P = inst[k].P;
-        P.parity = parity;
+        const StepParams& P = inst[k].P;
         double dt, ch, damp;
         if (!step_scalars(P, dt, ch, damp)) {
             if (local == 0 && lead) clock_flag_skip(P);
@@ -102,7 +101,7 @@ __global__ void __launch_bounds__(32 * YS_WARPS, PH::kYBlocks) batch_y_kernel(co
             y_march<PH>(T, inst[k].U, P, dt, ch, damp, strip, T.ng + r0, min(seg, T.ny - r0), vmax, reverts,
                         carry + threadIdx.y * YCarry<PH>::kSlots * 32);
         y_fold(P, vmax, reverts);
-        if (local == 0 && lead) clock_advance(P, dt, ch);
+        if (local == 0 && lead) clock_advance(P);
     }
 }
 
@@ -133,9 +132,9 @@ struct BatchLaunch {
         const cudaError_t attr = bx_setup<PH>();
         if (attr != cudaSuccess || which == 0) return attr;  // which 0: the set-up alone
         if (which == 1) {
-            batch_x_kernel<PH><<<ctas, 32 * BX_WARPS, bx_smem_bytes<PH>(), st>>>(inst, first, n, parity, xrpw);
+            batch_x_kernel<PH><<<ctas, 32 * BX_WARPS, bx_smem_bytes<PH>(), st>>>(inst + parity * n, first, n, xrpw);
         }
-        else batch_y_kernel<PH><<<ctas, dim3(32, YS_WARPS), 0, st>>>(inst, first + n + 1, n, parity, yseg);
+        else batch_y_kernel<PH><<<ctas, dim3(32, YS_WARPS), 0, st>>>(inst + parity * n, first + n + 1, n, yseg);
         return cudaGetLastError();
     }
 };

@@ -51,7 +51,7 @@ struct mhd_batch {
     std::vector<mhd_instance_desc> desc;
     std::vector<mhd_grid> U, T;
     std::vector<double> ch;  // per-instance c_h carried between runs (floor of the next CFL maximum)
-    std::vector<mhd::BatchInst> host_inst;
+    std::vector<mhd::BatchInst> host_inst;  // 2 n: step parity 0, then 1
     std::vector<int> first;  // x prefix (n + 1) then y prefix (n + 1)
     mhd::BatchInst* d_inst = nullptr;
     int* d_first = nullptr;
@@ -95,8 +95,12 @@ int build_worklist(mhd_batch* b) {
         b->first[i + 1] = b->first[i] + (int)(((long long)I.x_segs * b->desc[i].ny + mhd::BX_WARPS - 1) / mhd::BX_WARPS);
         b->first[b->n + 1 + i + 1] = b->first[b->n + 1 + i] + I.y_units;
     }
-    BCK(cudaMemcpyAsync(b->d_inst, b->host_inst.data(), sizeof(mhd::BatchInst) * b->n, cudaMemcpyHostToDevice,
-                        b->stream));
+    for (int i = 0; i < b->n; ++i) {
+        b->host_inst[b->n + i] = b->host_inst[i];
+        b->host_inst[b->n + i].P.parity = 1;
+    }
+    BCK(cudaMemcpyAsync(b->d_inst, b->host_inst.data(), sizeof(mhd::BatchInst) * b->host_inst.size(),
+                        cudaMemcpyHostToDevice, b->stream));
     BCK(cudaMemcpyAsync(b->d_first, b->first.data(), sizeof(int) * b->first.size(), cudaMemcpyHostToDevice,
                         b->stream));
     BCK(cudaStreamSynchronize(b->stream));
@@ -157,7 +161,7 @@ int mhd_batch_create(const mhd_instance_desc* desc, int n, int dtype, int solver
     b->U.assign(n, mhd_grid{});
     b->T.assign(n, mhd_grid{});
     b->ch.assign(n, 0.0);
-    b->host_inst.assign(n, mhd::BatchInst{});
+    b->host_inst.assign(2 * (size_t)n, mhd::BatchInst{});
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&b->nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -170,7 +174,7 @@ int mhd_batch_create(const mhd_instance_desc* desc, int n, int dtype, int solver
         if (!rc) rc = mhd_grid_alloc(&b->T[i], d.nx, d.ny, d.ng, dtype, d.x_min, d.x_max, d.y_min, d.y_max);
         b->cells += (long long)d.nx * d.ny;
     }
-    if (!rc && (cudaMalloc(&b->d_inst, sizeof(mhd::BatchInst) * n) != cudaSuccess ||
+    if (!rc && (cudaMalloc(&b->d_inst, sizeof(mhd::BatchInst) * 2 * n) != cudaSuccess ||
                 cudaMalloc(&b->d_first, sizeof(int) * 2 * (n + 1)) != cudaSuccess ||
                 cudaMalloc(&b->d_clock, sizeof(mhd::DevClock) * n) != cudaSuccess ||
                 cudaMalloc(&b->d_max, sizeof(unsigned long long) * n) != cudaSuccess))
@@ -193,6 +197,7 @@ int mhd_batch_create(const mhd_instance_desc* desc, int n, int dtype, int solver
         P.dy = (d.y_max - d.y_min) / d.ny;
         P.dmin = (P.dy < P.dx) ? P.dy : P.dx;
         P.t_end = d.t_end;
+        P.dt_min = 1.0e-8 * d.t_end;
         P.clock = b->d_clock + i;
         P.solver = solver;
         P.limiter = limiter;

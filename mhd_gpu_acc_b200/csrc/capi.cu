@@ -608,6 +608,7 @@ static int start_device_loop(mhd_workspace* ws, mhd_grid* U, mhd_grid* T, double
     *P = base_params(ws, U, solver, bc);
     P->cfl = cfl;
     P->t_end = t_end;
+    P->dt_min = 1.0e-8 * t_end;
     P->clock = ws->d_clock;
     P->accumulate = 1;
     return MHD_OK;
@@ -654,6 +655,7 @@ int mhd_sweep_clocked(mhd_workspace* ws, const mhd_grid* in, mhd_grid* out, int 
     mhd::StepParams P = base_params(ws, in, solver, bc);
     P.cfl = ws->clk_cfl;
     P.t_end = ws->clk_t_end;
+    P.dt_min = 1.0e-8 * ws->clk_t_end;
     P.clock = ws->d_clock;
     P.accumulate = 1;
     P.parity = parity;

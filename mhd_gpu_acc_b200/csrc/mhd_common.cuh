@@ -28,6 +28,7 @@ enum Solver : int { HLL = 0, HLLC = 1, HLLD = 2, FORCE = 3 };
 enum Limiter : int { MINMOD = 0, VANLEER = 1 };
 enum Bc : int { PERIODIC = 0, TRANSMISSIVE = 1, REFLECTING = 2, DIRICHLET = 3 };
 
+constexpr int kSMs = 148;  // streaming multiprocessors of one B200
 constexpr int MAX_NG = 4;  // ghost layers supported by the kernels (>= 2 needed)
 
 #ifdef __CUDACC__
@@ -79,13 +80,14 @@ struct DevClock {
     int status;          // 0 running, else one of ClockStatus
     unsigned int lowbeta_hits;   // FP32-bulk: FP64 pressure-recovery branch count
     unsigned int flux_fallbacks; // cells reverted by the non-finite update guard
+    double* log;         // {dt, ch, damp} of each step taken, when non-null
 };
 
 enum ClockStatus : int {
     CLK_OK = 0,
     CLK_NO_SPEED = 1,     // max wave speed <= 0 (the reference throws, solver_cpu.cpp:304-306)
     CLK_BAD_DT = 2,       // dt non-finite or <= 0 (scripts/cpu/main_cpu.cpp:205-209)
-    CLK_TINY_DT = 3,      // dt < 1e-8 t_end (scripts/cpu/main_cpu.cpp:210-216)
+    CLK_TINY_DT = 3,      // dt < dt_min, 1e-8 t_end (scripts/cpu/main_cpu.cpp:210-216)
     CLK_DONE = 8,         // t reached t_end: later steps of a captured loop are no-ops
     CLK_TIMEOUT = 16,     // a bounded device wait gave up
 };
@@ -98,6 +100,7 @@ struct StepParams {
     double dx, dy;
     double dmin;      // min(dx, dy)
     double t_end;
+    double dt_min;    // a device-mode step with a smaller dt is not taken: 1e-8 t_end
     // explicit mode (clock == nullptr): dt, ch and the psi damping factor
     double dt, ch, damp;
     DevClock* clock;  // device mode when non-null
@@ -142,9 +145,16 @@ __device__ __forceinline__ bool step_scalars(const StepParams& P, double& dt, do
     const double rem = P.t_end - t;
     dt = (rem < dt_raw) ? rem : dt_raw;
     if (!isfinite(dt) || dt <= 0.0) return false;
-    if (dt < 1.0e-8 * P.t_end) return false;
+    if (dt < P.dt_min) return false;
     damp = exp(-dt * ch / P.cr);
     return true;
+}
+
+// The step's c_h again, for a use after a march (the y-sweep runs at its register
+// limit: a double held across the march spills).
+__device__ __forceinline__ double step_ch(const StepParams& P) {
+    if (P.clock == nullptr) return P.ch;
+    return __longlong_as_double((long long)*(volatile const unsigned long long*)&P.clock->maxbits[P.parity]);
 }
 
 // Status for a skipped device-mode step (called by one thread).
@@ -159,7 +169,7 @@ __device__ __forceinline__ void clock_flag_skip(const StepParams& P) {
     const double rem = P.t_end - t;
     const double dt = (rem < dt_raw) ? rem : dt_raw;
     if (!isfinite(dt) || dt <= 0.0) { c->status = CLK_BAD_DT; return; }
-    if (dt < 1.0e-8 * P.t_end) { c->status = CLK_TINY_DT; return; }
+    if (dt < P.dt_min) { c->status = CLK_TINY_DT; return; }
 }
 
 // ---------------------------------------------------------------------------

@@ -503,7 +503,7 @@ __device__ __forceinline__ void y_segment(const DevGrid& in, const DevGrid& out,
         }
     }
     if (P.accumulate) {
-        const double v = PH::speed_of(acc, ch);
+        const double v = PH::speed_of(acc, step_ch(P));
         vmax = (vmax < v) ? v : vmax;
     }
 }
@@ -606,7 +606,7 @@ __device__ __forceinline__ void y_segment_carried(const DevGrid& in, const DevGr
         }
     }
     if (P.accumulate) {
-        const double v = PH::speed_of(acc, ch);
+        const double v = PH::speed_of(acc, step_ch(P));
         vmax = (vmax < v) ? v : vmax;
     }
 }
@@ -641,8 +641,16 @@ __device__ __forceinline__ void y_fold(const StepParams& P, double vmax, unsigne
 }
 
 // Clock advance of a completed device-mode step (one thread per step).
-__device__ __forceinline__ void clock_advance(const StepParams& P, double dt, double ch) {
+// The scalars are formed again rather than held across the march, which runs at
+// its register limit; the slots they come from do not change during the step.
+__device__ __forceinline__ void clock_advance(const StepParams& P) {
     DevClock* c = P.clock;
+    double dt, ch, damp;
+    step_scalars(P, dt, ch, damp);
+    if (c->log) {
+        double* l = c->log + 3 * c->steps;
+        l[0] = dt; l[1] = ch; l[2] = damp;
+    }
     c->t[P.parity ^ 1] = c->t[P.parity] + dt;
     c->steps += 1;
     c->last_dt = dt;
@@ -680,7 +688,7 @@ __global__ void __launch_bounds__(32 * PH::kYWarps, PH::kYBlocks) sweep_y_kernel
         y_march<PH>(in, out, P, dt, ch, damp, strip, in.ng + P.row0 + r0, count, vmax, reverts,
                     carry + threadIdx.y * YCarry<PH>::kSlots * 32);
     y_fold(P, vmax, reverts);
-    if (P.clock && first && !P.no_advance) clock_advance(P, dt, ch);
+    if (P.clock && first && !P.no_advance) clock_advance(P);
 }
 
 // Standalone CFL maximum over the interior (compute_dt, src/cpu/solver_cpu.cpp:283-303)

@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(32 * YT_WARPS, PH::kYTBlocks)
         y_band_tma<PH>(&map, in, out, P, dt, ch, damp, (blockIdx.x % groups) * YT_COLS, in.ng + r0,
                        min(per, row_end - r0), yt_smem, vmax, reverts);
     y_fold(P, vmax, reverts);
-    if (P.clock && first && !P.no_advance) clock_advance(P, dt, ch);
+    if (P.clock && first && !P.no_advance) clock_advance(P);
 }
 
 }  // namespace mhd
