@@ -114,7 +114,7 @@ __global__ void step_scalars_kernel(const double* sc, const double* log, int n1,
 // wave vector (mx, my) is sin(2 pi (mx x + my y)) / |(mx, my)|: with x fixed for
 // a thread that walks down a column, a cell costs one sincos of y (sums and
 // doubled angles give the eight modes) instead of eight sines, and a CTA adds
-// its 16 sums once: 127 -> 11 us at 512^2 FP32.
+// its 16 sums once: 127 -> 14 us at 512^2 FP32.
 constexpr int IC_ROWS = 8;
 template <typename R>
 __global__ void __launch_bounds__(256) ic_grad_kernel(DevGrid lam, DevGrid U0, double x0, double y0, double dx,

@@ -1,8 +1,8 @@
 // dispatch.cuh -- runtime (solver, limiter) -> template instance dispatch and
 // launch geometry of the two sweeps, shared by the FP64 and FP32 translation
 // units.  `which` selects the sweeps: 1 = x only, 2 = y only, 3 = both;
-// `yband` is the height of a y-sweep warp's row band and `xrpw` the x-sweep rows
-// per warp.
+// `yband` is the height of a y-sweep warp's row band and `xrpw` the x-sweep work
+// per warp (0: by the size of the launch, x_plan_auto / y_plan_auto).
 #pragma once
 
 #include "launch.h"
@@ -68,8 +68,10 @@ cudaError_t launch_policy(const DevGrid& in, const DevGrid& tmp, const DevGrid& 
     }
     if (which & 1) {
         // xrpw sets the x-sweep work per warp: row segments of 4 * xrpw chunks of 32 cells (then shorter
-        // ones); 0 = the policy's kXRpw
-        const SweepPlan pl = x_plan(in.nx, 4 * (xrpw > 0 ? xrpw : PH::kXRpw));
+        // ones); 0 = by the size of the launch, at most the policy's kXRpw
+        const SweepPlan pl = xrpw > 0 ? x_plan(in.nx, 4 * xrpw)
+                                      : x_plan_auto(in.nx, in.ny, kSMs * PH::kXBlocks * PH::kXWarps, PH::kXTask,
+                                                    4 * PH::kXRpw);
         const long long ctas = (plan_tasks(pl, in.ny) + PH::kXWarps - 1) / PH::kXWarps;
         sweep_x_kernel<PH><<<(unsigned)ctas, 32 * PH::kXWarps, x_smem_bytes<PH>(), st>>>(in, tmp, P, pl);
     }
@@ -85,7 +87,9 @@ cudaError_t launch_policy(const DevGrid& in, const DevGrid& tmp, const DevGrid& 
             sweep_y_tma_kernel<PH><<<(unsigned)(groups * bands), dim3(32, YT_WARPS), yt_smem_bytes<R>(), st>>>(
                 map, tmp, out, P, per);
         } else {
-            const SweepPlan pl = y_plan(rows, per);
+            const SweepPlan pl = yband > 0 ? y_plan(rows, yband)
+                                           : y_plan_auto(rows, y_strips(tmp), kSMs * PH::kYBlocks * PH::kYWarps,
+                                                         PH::kYTask, PH::kYBand);
             const long long warps = plan_tasks(pl, y_strips(tmp));
             const unsigned grid = (unsigned)((warps + PH::kYWarps - 1) / PH::kYWarps);
             sweep_y_kernel<PH><<<grid, dim3(32, PH::kYWarps), 0, st>>>(tmp, out, P, pl);

@@ -31,21 +31,23 @@ struct FastPolicy {
     static constexpr bool kYURing = true;
     static constexpr int kYBlocks = 4;  // y-sweep CTAs per SM the register budget is cut for
     static constexpr int kYTBlocks = 3; // the same for the TMA-staged y-sweep
-    // Default y band (rows one warp marches; shorter bands at the end of the
-    // launch, y_plan).  Measured at 4096^2 (HLLD, van Leer) with the guided
+    // Longest default y band (rows one warp marches; shorter bands at the end
+    // of the launch, y_plan; smaller launches take shorter bands, y_plan_auto).  Measured at 4096^2 (HLLD, van Leer) with the guided
     // phases: 28 rows 0.566 ms, 24 rows 0.567, 32 rows 0.586 (before the CFL
     // fold skip), 20 rows 0.594 (the same); with one band height: 24 rows
     // 0.659 ms, 16 rows 0.664, 32 rows 0.667, 48 rows 0.698.
     static constexpr int kYBand = 28;
+    static constexpr double kYTask = 1.85;  // y_plan_auto's factor
     // x-sweep (row march, segments of 1020 cells): 4 warps per CTA, 4 CTAs per
     // SM (128 registers, 56 KB of rings per CTA).  Measured at 4096^2 (HLLD, van
     // Leer): 0.549 ms; segments of 508 cells 0.545 ms, of 2044 cells 0.588 ms.
     // (The lane-per-cell tile it replaced: 0.574 ms.)
     static constexpr int kXWarps = 4;
     static constexpr int kXBlocks = 4;
-    // Default x work per warp: segments of 1020 cells (the last quarter of a
+    // Largest default x work per warp (smaller launches: x_plan_auto): segments of 1020 cells (the last quarter of a
     // row in 316-cell ones); 2044-cell segments measured 0.520 ms, 508-cell 0.551.
     static constexpr int kXRpw = 8;
+    static constexpr double kXTask = 2.2;  // x_plan_auto's factor
     // Reloading the updated cell at the top of each x-march step needs 9 more
     // registers across the solve: at 128 registers that spills, and measured
     // 0.576 ms against 0.549 ms for the reload just before the update.

@@ -30,13 +30,15 @@ struct ExactPolicy {
     static constexpr bool kYURing = false;
     static constexpr int kYBlocks = 2;  // y-sweep CTAs per SM the register budget is cut for
     static constexpr int kYTBlocks = 2; // the same for the TMA-staged y-sweep
-    // Default y band (shorter bands at the end of the launch, y_plan).
+    // Longest default y band (shorter bands at the end of the launch, y_plan;
+    // smaller launches take shorter bands, y_plan_auto).
     // Measured at 4096^2 (HLLD, van Leer) with the guided phases and the fold
     // skip: 56 rows 2.62 ms, 48 rows 2.63, 64 rows 2.63, 80 rows 2.64, 40 rows
     // 2.65, 32 rows 2.68, 128 rows 2.89 (FP32 runs fastest at 28: its faster
     // sweep is the more sensitive to the DRAM locality of short bands); with
     // one band height: 32 rows 2.97 ms, 24 rows 2.98, 48 rows 2.98.
     static constexpr int kYBand = 56;
+    static constexpr double kYTask = 2.2;  // y_plan_auto's factor
     // x-sweep (row march): 4 warps per CTA, 2 CTAs per SM (238 registers, no
     // spills), the updated cell reloaded at the top of each step.  Measured at
     // 4096^2 (HLLD, van Leer): 2.21 ms, against 2.27 ms reloading just before
@@ -49,10 +51,11 @@ struct ExactPolicy {
     // not made; 2 CTAs x 80 KB of rings): measured at 4096^2 2.174 -> 2.147 ms
     // (step 4.795 -> 4.766 ms), bit-identical results.
     static constexpr bool kXURing = true;
-    // Default x work per warp: segments of 2044 cells (the last quarter of a
+    // Largest default x work per warp (smaller launches: x_plan_auto): segments of 2044 cells (the last quarter of a
     // row in 668-cell ones).  Measured at 4096^2: 2.175 ms, against 2.210 ms
     // for 1020-cell segments.
     static constexpr int kXRpw = 16;
+    static constexpr double kXTask = 2.8;  // x_plan_auto's factor
     struct Prim { double v[NV]; };
     struct Side { double v[NV]; };
 

@@ -388,8 +388,9 @@ __host__ __device__ __forceinline__ bool plan_task(const SweepPlan& pl, long lon
     const int lo = p0 ? pl.lo[0] : (p1 ? pl.lo[1] : pl.lo[2]);
     const int hi = p0 ? pl.lo[1] : (p1 ? pl.lo[2] : pl.lo[3]);
     const int l = p0 ? pl.len[0] : (p1 ? pl.len[1] : pl.len[2]);
-    idx = (int)(k % width);
-    start = lo + (int)(k / width) * l;
+    const unsigned t = (unsigned)k;  // tasks of one launch: under 2^32
+    idx = (int)(t % (unsigned)width);
+    start = lo + (int)(t / (unsigned)width) * l;
     len = min(l, hi - start);
     return true;
 }
@@ -415,6 +416,44 @@ __host__ __device__ inline SweepPlan x_plan(int nx, int chunks) {
 __host__ __device__ inline SweepPlan y_plan(int rows, int per) {
     const int p1 = per / 2 > 1 ? per / 2 : 1, p2 = per / 4 > 1 ? per / 4 : 1;
     return guided_plan(rows, per, p1, p2, kYPhase0End, kYPhase1End);
+}
+
+// Task length by the size of the launch.  With `work` = warp iterations (x:
+// 32-cell chunks, y: rows of a strip) and `slots` resident warps, N = work /
+// slots iterations fall to each slot.  Long tasks waste least (every task
+// repeats a two-cell / two-row halo, so the repeated work falls as N / len),
+// but the launch ends on stragglers of one task's length: the sum is least at
+// len ~ sqrt(N), with the factor `c` measured per sweep and precision and `cap`
+// the longest worth taking (the large-grid lengths, kXRpw and kYBand).  Up to
+// `one_wave` iterations per slot the tasks all run at once, and the shortest
+// length that still fits them in one wave is best (x: 4, y: 8; e.g. FP32 y at
+// 512^2, N = 3.7: 53 / 38 / 37 / 31 / 33 / 36 us with 1 / 2 / 3 / 4 / 5 / 6
+// rows).  Measured (HLLD, van Leer, us; with the cap's length at every size ->
+// by this rule): FP32 x 512^2 35 -> 22, 1024^2 55 -> 48, y 512^2 107 -> 31,
+// 1024^2 121 -> 72, 2048^2 202 -> 183; FP64 x 512^2 64 -> 55, 1024^2 173 -> 160,
+// y 512^2 445 -> 91, 1024^2 454 -> 235, 2048^2 781 -> 687; 64^2 y 106 -> 14 FP32,
+// 423 -> 23 FP64.
+constexpr double kXOneWave = 4.0, kYOneWave = 8.0;
+struct TaskLen {
+    int len;
+    bool one_wave;  // equal tasks, no guided tail
+};
+inline TaskLen task_len(long long work, int slots, double c, int cap, double one_wave) {
+    const double n = (double)work / slots;
+    const bool one = n <= one_wave;
+    const double len = one ? std::ceil(n) : std::floor(c * std::sqrt(n) + 0.5);
+    return {len < 1.0 ? 1 : (len > cap ? cap : (int)len), one};
+}
+
+// The x- / y-sweep plan of a launch whose caller leaves the shape open.
+inline SweepPlan x_plan_auto(int nx, int rows, int slots, double c, int cap_chunks) {
+    const TaskLen t = task_len((long long)rows * ((nx + 31) / 32), slots, c, cap_chunks, kXOneWave);
+    const int len = x_seg_len(t.len);
+    return t.one_wave ? guided_plan(nx, len, len, len, 64, 64) : x_plan(nx, t.len);
+}
+inline SweepPlan y_plan_auto(int rows, int strips, int slots, double c, int cap_rows) {
+    const TaskLen t = task_len((long long)rows * strips, slots, c, cap_rows, kYOneWave);
+    return t.one_wave ? guided_plan(rows, t.len, t.len, t.len, 64, 64) : y_plan(rows, t.len);
 }
 
 // CTA shape and register budget per policy: PH::kXWarps warps per CTA,
