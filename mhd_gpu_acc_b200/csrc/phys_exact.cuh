@@ -540,31 +540,5 @@ MHD_HD_INLINE double cell_speed(const double* U, double g, double ch) {
     return -1.0;
 }
 
-// cell_speed folded into a running maximum acc, skipping the fast speeds of a
-// cell whose speed provably stays under the floor ch: cell_speed returns
-// exactly ch for such a cell (both directional speeds are floored by it), so
-// the maximum is the same bit for bit.  The test needs no division: with
-// r = rho, r e = r E - (|m|^2 + r |B|^2) / 2 (rho times the internal energy)
-// and X = g (g - 1) r e + r |B|^2 = r^2 (a^2 + b^2), the speed is under
-// max(|u|, |v|) + sqrt(a^2 + b^2) = (max(|m_x|, |m_y|) + sqrt(X)) / r, as
-// c_f^2 = (s + sqrt(s^2 - 4 a^2 b_n^2)) / 2 <= s = a^2 + b^2.  Margins: the
-// internal energy above 1e-6 of |E| (c2p's pressure then is surely positive)
-// and the bound 1e-12 under ch (far above the rounding of either form).
-// Non-physical and non-finite cells take cell_speed.
-MHD_HD_INLINE void fold_cell_speed_floored(const double* U, double g, double ch, double& acc) {
-    const double r = U[RHO];
-    const double m2 = U[MX] * U[MX] + U[MY] * U[MY] + U[MZ] * U[MZ];
-    const double B2r = (U[BX] * U[BX] + U[BY] * U[BY] + U[BZ] * U[BZ]) * r;
-    const double re = U[EN] * r - 0.5 * (m2 + B2r);
-    const double X = g * (g - 1.0) * re + B2r;
-    const double mm = fmax(fabs(U[MX]), fabs(U[MY]));
-    if (r > 0.0 && re > 1.0e-6 * fabs(U[EN]) * r && mm + sqrt(X) < ch * r * (1.0 - 1.0e-12)) {
-        acc = (acc < ch) ? ch : acc;
-        return;
-    }
-    const double s = cell_speed(U, g, ch);
-    acc = (acc < s) ? s : acc;
-}
-
 }  // namespace exact
 }  // namespace mhd

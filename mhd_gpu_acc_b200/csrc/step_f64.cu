@@ -2,10 +2,11 @@
 // physics of phys_exact.cuh driven by the fused sweeps of sweep.cuh.
 //
 // Build this translation unit with --fmad=false: together with the reference
-// operand order in phys_exact.cuh it makes the GPU step reproduce the
-// reference's CPU/OpenMP FP64 step (src/cpu/solver_cpu.cpp) bit for bit.
+// operand order in phys_exact.cuh, whose values phys_exact_sweep.cuh forms, it
+// makes the GPU step reproduce the reference's CPU/OpenMP FP64 step
+// (src/cpu/solver_cpu.cpp) bit for bit.
 #include "launch.h"
-#include "phys_exact.cuh"
+#include "phys_exact_sweep.cuh"
 #include "dispatch.cuh"
 #include "batch.cuh"
 
@@ -15,13 +16,18 @@ template <int SOLVER, int LIMITER>
 struct ExactPolicy {
     using Real = double;
     static constexpr int NW = NV;  // primitive values per cell
-    static constexpr int NS = NV;  // values per reconstructed side state (U*)
-    static constexpr int NSY = NV;  // the same in the y-sweep's carried window
+    static constexpr int NS = 14;  // values per reconstructed side state (U*, its u, v, w, p and 1 / rho)
+    static constexpr int NSY = 14;  // the same in the y-sweep's carried window
     template <class S>
     __device__ static void y_side_rest(S&) {}
     static constexpr int kYWarps = 4;   // y-sweep warps per CTA (side by side)
+    // The face-side states carry their primitives and 1 / rho, and quotients and
+    // roots come in branch-free groups (phys_exact_sweep.cuh): at 4096^2 (HLLD, van
+    // Leer) x 2.044 -> 1.440 ms, y 2.373 -> 1.690 ms, at 2048^2 x 0.591 -> 0.395,
+    // y 0.687 -> 0.492 ms, bit-identical results.  The kernels wait on FP64
+    // latency (2 warps per scheduler, FP64 pipe 50 % busy, 37 % before).
     // y-sweep window in shared memory (y_segment_carried), 2 CTAs per SM.
-    // Measured at 4096^2 (HLLD, van Leer): 2.97 ms, against 3.11 ms for the
+    // Measured before that at 4096^2 (HLLD, van Leer): 2.97 ms, against 3.11 ms for the
     // register window (255 registers, spills) and 3.06 ms for the shared-memory
     // window at 3 CTAs (168 registers, spills).
     static constexpr bool kYCarry = true;
@@ -57,28 +63,25 @@ struct ExactPolicy {
     static constexpr int kXRpw = 16;
     static constexpr double kXTask = 2.8;  // x_plan_auto's factor
     struct Prim { double v[NV]; };
-    struct Side { double v[NV]; };
+    using Side = exact::Side;
 
-    __device__ static void prim(const double* U, double g, double* W) { exact::c2p(U, g, W); }
+    __device__ static void prim(const double* U, double g, double* W) { exact::c2p_grouped(U, g, W); }
     // A face-side state made directly from a conserved cell (the solvers' input).
     template <int DIR>
-    __device__ static void side(const double* U, double, Side& S) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) S.v[k] = U[k];
-    }
+    __device__ static void side(const double* U, double g, Side& S) { exact::side_of(U, g, S); }
 
     template <int DIR>
     __device__ static void recon(const Prim& Wm, const Prim& Wc, const Prim& Wp, double dtd, double ch, double g,
                                  Side& L, Side& R) {
-        exact::reconstruct<DIR, LIMITER>(Wm.v, Wc.v, Wp.v, dtd, ch, g, L.v, R.v);
+        exact::reconstruct_of<DIR, LIMITER>(Wm.v, Wc.v, Wp.v, dtd, ch, g, L, R);
     }
 
     template <int DIR>
     __device__ static void face(const Side& Rl, const Side& Lr, double ch, double g, double* F) {
-        exact::riemann<DIR, SOLVER>(Rl.v, Lr.v, ch, g, F);
+        exact::riemann_of<DIR, SOLVER>(Rl, Lr, ch, g, F);
     }
 
-    __device__ static double speed(const double* U, double g, double ch) { return exact::cell_speed(U, g, ch); }
+    __device__ static double speed(const double* U, double g, double ch) { return exact::cell_speed_of(U, g, ch); }
 
     // The y-sweep's running CFL maximum (cell_speed per cell, as the reference;
     // the fast speeds of cells provably under the floor ch are skipped, which
@@ -86,7 +89,7 @@ struct ExactPolicy {
     using SpeedAcc = double;
     __device__ static SpeedAcc no_speed() { return 0.0; }
     __device__ static void fold_speed(const double* U, double g, double ch, SpeedAcc& acc) {
-        exact::fold_cell_speed_floored(U, g, ch, acc);
+        exact::fold_cell_speed(U, g, ch, acc);
     }
     __device__ static double speed_of(SpeedAcc acc, double) { return acc; }
 };
