@@ -312,8 +312,8 @@ int mhd_initialise_device(mhd_workspace* ws, const mhd_grid* g, int case_id);
 int mhd_initialise_orszag_tang(mhd_workspace* ws, const mhd_grid* g, double b0, double gamma, const double* amp);
 
 /* ---- batched instances (no reference counterpart) ----
- * Many independent problems of uneven size advanced together: one persistent
- * launch per sweep phase over a global tile work list, CUDA-graph step loop,
+ * Many independent problems of uneven size advanced together: one launch per
+ * sweep phase over a global work list, CUDA-graph step loop,
  * per-instance gamma, CFL, c_r, boundary types, t_end, dt and c_h.  Solver,
  * limiter and precision are shared.  Dirichlet sides are not supported. */
 typedef struct mhd_instance_desc {
@@ -324,7 +324,8 @@ typedef struct mhd_instance_desc {
 } mhd_instance_desc;
 /* Launch shape of the batched sweeps: x-sweep work per warp (xrpw: row
  * segments of 128 * xrpw - 4 cells), y-sweep segment length, persistent CTAs
- * of each phase (0 = default from the SM count). */
+ * of each phase (0 = default from the SM count).  A batch that was never tuned
+ * takes the lengths that suit its size and deals the work out dynamically. */
 typedef struct mhd_batch_tuning {
     int xrpw, yseg, ctas_x, ctas_y;
 } mhd_batch_tuning;
@@ -346,8 +347,9 @@ int mhd_batch_get_tuning(const mhd_batch* b, mhd_batch_tuning* t);
 int mhd_batch_set_tuning(mhd_batch* b, const mhd_batch_tuning* t);
 /* Autotuner: times each sweep phase for every candidate launch shape (x work
  * per warp xrpw 2/4/8/16 x 2-4 CTAs per SM; y segment 16/24/32/48/64/128 x 2-4
- * CTAs per SM) on the batch's current states, `reps` launches each, and keeps
- * the fastest.  Leaves the instances one step ahead. */
+ * CTAs per SM) on the batch's current states, `reps` launches each, and the
+ * untuned shape, and keeps the fastest of each phase (*best: the fastest
+ * candidate).  Leaves the instances one step ahead. */
 int mhd_batch_tune(mhd_batch* b, int reps, mhd_batch_tuning* best);
 /* The autotuner's candidate values: which = 0 x work per warp (xrpw), 1 y
  * segment lengths, 2 CTAs per SM (both phases).  Copies up to cap of them into

@@ -1,17 +1,24 @@
 // batch.cuh -- many independent instances of uneven size advanced together.
 //
 // Each instance (its own grid, gamma, CFL, c_r, boundary types, t_end and
-// device clock) is cut into the same work units the single-grid sweeps use:
-// x units of BX_WARPS (row, segment) tasks, segments of x_seg_len(4 * rpw)
-// cells marched by one warp each (x_segment); y units of YS_WARPS
-// consecutive (strip, band) items of an instance, strip-fastest (a strip is 32
-// columns, a band seg rows), as the single-grid y-sweep orders its warps.  The units of all instances
-// form one global list (prefix offsets in `first`, split by phase: first[0..n]
-// for x, first[n+1..2n+1] for y).  A persistent launch per sweep phase -- `ctas` CTAs striding over the
-// list -- advances every instance; the kernel boundary between the x and y
-// phases is the only synchronisation a step needs, and a CUDA graph of two
-// steps replays the loop.  Instance k's unit 0 performs the clock duties the
-// single-grid kernels give to CTA (0, 0).
+// device clock) is cut into the same tasks the single-grid sweeps use: row
+// segments marched by one warp each (x_segment) and row bands of 32-column
+// strips (y_march), in equal lengths up to the longest that suits the size of the
+// whole batch, the last eighth of its rows in a third of that.  Four consecutive
+// tasks of one instance and length form a unit, the work of one CTA.  The units
+// of all instances form one global list, longest tasks first, so that the launch
+// ends on short ones; a table gives each unit's segment (one per instance and
+// length).  One launch per sweep phase advances every instance; the kernel
+// boundary between the x and y phases is the only synchronisation a step needs,
+// and a CUDA graph of two steps replays the loop.
+// The first unit of an instance performs the clock duties the single-grid
+// kernels give to CTA (0, 0).
+//
+// By default a CTA takes one unit and the hardware deals them out: at 96
+// instances of 64..1024 cells a side (29.5M cells, FP32 HLLD, van Leer) x 1.21 ->
+// 0.89 ms and y 1.99 -> 1.19 ms against 444 CTAs striding over the list in fixed
+// order with one task length (kDefaultBatchXRpw, kDefaultYSeg; of the y gain 0.2 ms
+// is the ghost scatter's).  An explicit tuning keeps that form.
 #pragma once
 
 #include "dispatch.cuh"
@@ -21,87 +28,143 @@ namespace mhd {
 constexpr int BX_WARPS = 4;  // warps per batched x-sweep CTA
 
 // The device table holds every instance twice, with P.parity 0 and then 1, so that
-// the kernels read an instance's parameters where they lie instead of copying
-// them per thread.
+// the kernels can read an instance's parameters where they lie.
 struct BatchInst {
-    DevGrid U, T;
+    DevGrid U;
+    void* T;       // the x-swept state, of U's layout
     StepParams P;  // physics, boundary types, t_end, clock and step parity of this instance
-    int x_segs, x_pad_;      // x-sweep segments per row
-    int y_strips, y_bands;   // 32-column strips; bands of seg rows
-    int y_units;             // ceil(strips * bands / YS_WARPS)
-    int pad_;
 };
 
-// largest k in [0, n) with first[k] <= u (first is non-decreasing, first[0] = 0)
-__device__ __forceinline__ int find_instance(const int* first, int n, int u) {
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(first + mid) <= u) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
+// n tasks of `len` cells (the last may be shorter) per row / strip, covering
+// [lo, hi) of each of the `width` rows (x) or strips (y) from idx0 on of an
+// instance; `lead`: the segment's first unit (`unit` of the list) does the
+// instance's clock duties.
+struct BatchSeg {
+    int inst, lo, hi, len, n, idx0, width, lead, unit;
+};
+
+// Task `task` of a segment: false past its last.
+__device__ __forceinline__ bool seg_task(const BatchSeg& s, int task, int& idx, int& start, int& len) {
+    if (task >= s.n * s.width) return false;
+    idx = s.idx0 + task % s.width;
+    start = s.lo + task / s.width * s.len;
+    len = min(s.len, s.hi - start);
+    return true;
 }
 
 // Dynamic shared memory of the batched x-sweep: one x_segment ring per warp.
 template <class PH>
 constexpr int bx_smem_bytes() { return BX_WARPS * XRing<PH>::kWarpBytes; }
 
-template <class PH>
-__global__ void __launch_bounds__(32 * BX_WARPS, PH::kXBlocks) batch_x_kernel(const BatchInst* __restrict__ inst,
-                                                              const int* __restrict__ first, int n, int rpw) {
+// STRIDE: the CTAs stride over the list (an explicit tuning); else CTA u takes unit
+// u, which leaves the march the loop's registers (without them it spills 8 bytes:
+// 908 -> 892 us at 96 instances of 64..1024 cells a side).
+template <class PH, bool STRIDE>
+__global__ void __launch_bounds__(32 * BX_WARPS, PH::kXBlocks)
+    batch_x_kernel(const BatchInst* __restrict__ inst, const BatchSeg* __restrict__ seg, const int* __restrict__ unit_seg,
+                   int total) {
     using V = typename Slot16<typename PH::Real>::V;
     extern __shared__ __align__(16) unsigned char bx_smem[];
     const int warp = threadIdx.x >> 5;
     V* ring = reinterpret_cast<V*>(bx_smem + warp * XRing<PH>::kWarpBytes);
-    const int len = x_seg_len(4 * rpw);
-    const int total = __ldg(first + n);
-    for (int u = blockIdx.x; u < total; u += gridDim.x) {
-        const int k = find_instance(first, n, u);
-        const int local = u - __ldg(first + k);
-        const StepParams& P = inst[k].P;
+    for (int u = blockIdx.x; u < total; u = STRIDE ? u + gridDim.x : total) {
+        const BatchSeg s = seg[__ldg(unit_seg + u)];
+        const int local = u - s.unit;
+        const bool lead = s.lead && local == 0 && threadIdx.x == 0;
+        const StepParams& P = inst[s.inst].P;
         double dt, ch, damp;
         if (!step_scalars(P, dt, ch, damp)) {
-            if (local == 0 && threadIdx.x == 0) clock_flag_skip(P);
+            if (lead) clock_flag_skip(P);
             continue;
         }
-        if (local == 0 && threadIdx.x == 0) P.clock->maxbits[P.parity ^ 1] = 0ull;
-        const DevGrid& U = inst[k].U;
-        const long long task = (long long)local * BX_WARPS + warp;
-        if (task < (long long)inst[k].x_segs * U.ny) {  // whole warp
-            const int row = (int)(task % U.ny), c0 = (int)(task / U.ny) * len;
-            x_segment<PH>(U, inst[k].T, P, dt, ch, U.ng + row, c0, min(len, U.nx - c0), ring);
+        if (lead) P.clock->maxbits[P.parity ^ 1] = 0ull;
+        int row, c0, len;
+        if (seg_task(s, local * BX_WARPS + warp, row, c0, len)) {  // whole warp
+            const DevGrid in = inst[s.inst].U;
+            DevGrid out = in;
+            out.data = inst[s.inst].T;
+            x_segment<PH>(in, out, P, dt, ch, in.ng + row, c0, len, ring);
         }
     }
 }
 
 template <class PH>
-__global__ void __launch_bounds__(32 * YS_WARPS, PH::kYBlocks) batch_y_kernel(const BatchInst* __restrict__ inst,
-                                                               const int* __restrict__ first, int n, int seg) {
+__global__ void __launch_bounds__(32 * YS_WARPS, PH::kYBlocks)
+    batch_y_kernel(const BatchInst* __restrict__ inst, const BatchSeg* __restrict__ seg, const int* __restrict__ unit_seg,
+                   int total) {
     using R = typename PH::Real;
     __shared__ __align__(16) R carry[PH::kYCarry ? YS_WARPS * YCarry<PH>::kSlots * 32 : 1];
-    const int total = __ldg(first + n);
-    const bool lead = (threadIdx.x == 0 && threadIdx.y == 0);
+    // The instance in shared memory, read where it is used: held in registers (as
+    // the single-grid sweep holds nothing, its parameters being constants) it
+    // makes the march spill, and spills miss in the L1 that the windows leave.
+    __shared__ BatchInst I;
+    __shared__ DevGrid T;
     for (int u = blockIdx.x; u < total; u += gridDim.x) {
-        const int k = find_instance(first, n, u);
-        const int local = u - __ldg(first + k);
-        const StepParams& P = inst[k].P;
+        const BatchSeg s = seg[__ldg(unit_seg + u)];
+        const int local = u - s.unit;
+        const bool lead = s.lead && local == 0 && threadIdx.x == 0 && threadIdx.y == 0;
+        static_assert(sizeof(BatchInst) % 4 == 0 && sizeof(BatchInst) / 4 <= 32 * YS_WARPS, "copied a word per thread");
+        __syncthreads();  // the unit before may still be reading I
+        const int q = threadIdx.y * 32 + threadIdx.x;
+        if (q < (int)(sizeof(BatchInst) / 4)) reinterpret_cast<int*>(&I)[q] = reinterpret_cast<const int*>(&inst[s.inst])[q];
+        __syncthreads();
+        if (q == 0) {
+            T = I.U;
+            T.data = I.T;
+        }
+        __syncthreads();
+        const StepParams& P = I.P;
         double dt, ch, damp;
         if (!step_scalars(P, dt, ch, damp)) {
-            if (local == 0 && lead) clock_flag_skip(P);
+            if (lead) clock_flag_skip(P);
             continue;
         }
-        const int strips = inst[k].y_strips;
-        const DevGrid& T = inst[k].T;
-        const int item = local * YS_WARPS + threadIdx.y;
-        const int strip = item % strips, r0 = (item / strips) * seg;
         double vmax = 0.0;
         unsigned reverts = 0;
-        if (item < strips * inst[k].y_bands)
-            y_march<PH>(T, inst[k].U, P, dt, ch, damp, strip, T.ng + r0, min(seg, T.ny - r0), vmax, reverts,
+        int strip, r0, count;
+        if (seg_task(s, local * YS_WARPS + threadIdx.y, strip, r0, count)) {
+            y_march<PH>(T, I.U, P, dt, ch, damp, strip, T.ng + r0, count, vmax, reverts,
                         carry + threadIdx.y * YCarry<PH>::kSlots * 32);
+        }
         y_fold(P, vmax, reverts);
-        if (local == 0 && lead) clock_advance(P);
+        if (lead) clock_advance(P);
+    }
+}
+
+// CFL maximum of every instance (compute_dt's, floored by the instance's ch) into
+// maxbits[0] of its clock, which starts at 0: CTAs of 256 threads take
+// kMaxUnit cells of one instance each, one atomic per CTA.
+constexpr int kMaxUnit = 4096;
+template <class PH>
+__global__ void __launch_bounds__(256) batch_max_kernel(const BatchInst* __restrict__ inst,
+                                                       const BatchSeg* __restrict__ seg,
+                                                       const int* __restrict__ unit_seg,
+                                                       const double* __restrict__ ch) {
+    using R = typename PH::Real;
+    __shared__ double part[8];
+    const BatchSeg s = seg[__ldg(unit_seg + blockIdx.x)];
+    const BatchInst& I = inst[s.inst];
+    const DevGrid g = I.U;
+    const double gamma = I.P.gamma, floor_ch = ch[s.inst];
+    const int c0 = ((int)blockIdx.x - s.unit) * kMaxUnit, c1 = min(s.hi, c0 + kMaxUnit);
+    double vmax = 0.0;
+    for (int c = c0 + threadIdx.x; c < c1; c += 256) {
+        const int j = c / g.nx, i = c - j * g.nx;
+        R U[NV];
+        load_cell(g, g.ng + i, g.ng + j, U);
+        const double v = PH::speed(U, gamma, floor_ch);
+        vmax = (vmax < v) ? v : vmax;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double t = __shfl_xor_sync(FULL, vmax, o);
+        vmax = (vmax < t) ? t : vmax;
+    }
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = vmax;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) vmax = (vmax < part[w]) ? part[w] : vmax;
+        atomic_max_pos(&I.P.clock->maxbits[0], vmax);
     }
 }
 
@@ -113,37 +176,65 @@ cudaError_t bx_setup() {
                   "batched x-phase rings of kXBlocks CTAs exceed an SM's shared memory");
     static PerDeviceOnce once;
     return once.run([] {
-        cudaError_t r = cudaFuncSetAttribute(batch_x_kernel<PH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             bx_smem_bytes<PH>());
+        cudaError_t r = cudaSuccess;
+        for (auto* k : {batch_x_kernel<PH, false>, batch_x_kernel<PH, true>}) {
+            if (r == cudaSuccess) r = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bx_smem_bytes<PH>());
+            if (r == cudaSuccess)
+                r = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+        }
+        // the y phase's window and parameters are a little over the 40 KB of which
+        // four CTAs fit the 164 KB split that the runtime picks: ask for the next one,
+        // 196 of 228 KB (85 %; more leaves too little L1)
         if (r == cudaSuccess)
-            r = cudaFuncSetAttribute(batch_x_kernel<PH>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                     (int)cudaSharedmemCarveoutMaxShared);
+            r = cudaFuncSetAttribute(batch_y_kernel<PH>, cudaFuncAttributePreferredSharedMemoryCarveout, 85);
         return r;
     });
 }
 
+// One phase's work list.
+struct BatchList {
+    const BatchSeg* seg;
+    const int* unit_seg;  // the segment of each unit
+    int units;
+};
+
 struct BatchLaunch {
     const BatchInst* inst;
-    const int* first;
-    int n, parity, which, xrpw, yseg, ctas;
+    BatchList list;
+    int n, parity, which, ctas;
     cudaStream_t st;
     template <class PH>
     cudaError_t run() const {
         const cudaError_t attr = bx_setup<PH>();
         if (attr != cudaSuccess || which == 0) return attr;  // which 0: the set-up alone
-        if (which == 1) {
-            batch_x_kernel<PH><<<ctas, 32 * BX_WARPS, bx_smem_bytes<PH>(), st>>>(inst + parity * n, first, n, xrpw);
-        }
-        else batch_y_kernel<PH><<<ctas, dim3(32, YS_WARPS), 0, st>>>(inst + parity * n, first + n + 1, n, yseg);
+        const BatchInst* I = inst + parity * n;
+        const dim3 yb(32, YS_WARPS);
+        constexpr int smem = bx_smem_bytes<PH>();
+        const int grid = ctas > 0 ? ctas : list.units;
+        if (which == 2) batch_y_kernel<PH><<<grid, yb, 0, st>>>(I, list.seg, list.unit_seg, list.units);
+        else if (ctas > 0) batch_x_kernel<PH, true><<<grid, 32 * BX_WARPS, smem, st>>>(I, list.seg, list.unit_seg, list.units);
+        else batch_x_kernel<PH, false><<<grid, 32 * BX_WARPS, smem, st>>>(I, list.seg, list.unit_seg, list.units);
         return cudaGetLastError();
     }
 };
 
 template <template <int, int> class POL>
-cudaError_t dispatch_batch(const BatchInst* inst, const int* first, int n, int parity, int which, int solver,
-                           int limiter, int xrpw, int yseg, int ctas, cudaStream_t st) {
-    BatchLaunch go{inst, first, n, parity, which, xrpw, yseg, ctas, st};
+cudaError_t dispatch_batch(const BatchInst* inst, const BatchList& list, const double* ch, int n, int parity, int which,
+                           int solver, int limiter, int ctas, cudaStream_t st) {
+    if (which == 3) {
+        batch_max_kernel<POL<HLL, MINMOD>><<<list.units, 256, 0, st>>>(inst, list.seg, list.unit_seg, ch);
+        return cudaGetLastError();
+    }
+    BatchLaunch go{inst, list, n, parity, which, ctas, st};
     return with_policy<POL>(solver, limiter, go);
+}
+
+// Longest x and y tasks by the size of the whole batch (iterations of all
+// instances over the resident warps), as the single-grid sweeps take theirs.
+template <class PH>
+void batch_task_lens(long long x_work, long long y_work, TaskLen& x, TaskLen& y) {
+    x = task_len(x_work, kSMs * PH::kXBlocks * BX_WARPS, PH::kXTask, 4 * PH::kXRpw, kXOneWave);
+    y = task_len(y_work, kSMs * PH::kYBlocks * YS_WARPS, PH::kYTask, PH::kYBand, kYOneWave);
 }
 
 }  // namespace mhd

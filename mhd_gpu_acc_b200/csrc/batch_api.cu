@@ -2,16 +2,18 @@
 //
 // A batch owns, per instance, the state U and the x-swept state T (padded slabs
 // as mhd_grid_alloc makes them), a device clock, and one shared instance table
-// and work list (batch.cuh).  mhd_batch_run starts every clock from the CFL
-// maximum of its instance and replays a CUDA graph of two steps (four
-// persistent launches) until max_steps steps or every instance's t_end.
+// and work lists (batch.cuh).  mhd_batch_run starts every clock from the CFL
+// maximum of its instance (one launch for all) and replays a CUDA graph of two
+// steps (four launches) until max_steps steps or every instance's t_end.
 //
 // Autotuner (mhd_batch_tune): the x-sweep phase maps U -> T and the y-sweep
 // phase maps T -> U without touching the clock slots they read, so each phase
 // can be launched repeatedly on unchanged input.  The tuner times every x
 // candidate (rows per warp x persistent CTAs) and then every y candidate
-// (segment length x persistent CTAs) with CUDA events, keeping the fastest of
-// each.  The instances end one step ahead of where they started.
+// (segment length x persistent CTAs) with CUDA events, and the default shape by
+// the size of the batch, keeping the fastest of each phase.  The instances end one
+// step ahead of where they started.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -36,14 +38,6 @@ int berr(int code, const char* msg) { return mhd::report_error(code, msg); }
         if (e_ != cudaSuccess) return berr(MHD_ERR_CUDA, cudaGetErrorString(e_)); \
     } while (0)
 
-__global__ void batch_clock_init(mhd::DevClock* c, const unsigned long long* mx, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    mhd::DevClock z{};
-    z.maxbits[0] = mx[i];
-    c[i] = z;
-}
-
 }  // namespace
 
 struct mhd_batch {
@@ -52,15 +46,19 @@ struct mhd_batch {
     std::vector<mhd_grid> U, T;
     std::vector<double> ch;  // per-instance c_h carried between runs (floor of the next CFL maximum)
     std::vector<mhd::BatchInst> host_inst;  // 2 n: step parity 0, then 1
-    std::vector<int> first;  // x prefix (n + 1) then y prefix (n + 1)
     mhd::BatchInst* d_inst = nullptr;
-    int* d_first = nullptr;
+    // work lists of the x phase, the y phase and the CFL maximum: segments (up to
+    // 2 n each for x and y, n for the maximum) and the segment of every unit
+    mhd::BatchSeg* d_seg = nullptr;
+    int* d_units = nullptr;
+    size_t units_cap = 0;
+    mhd::BatchList lists[3] = {};
+    double* d_ch = nullptr;
     mhd::DevClock* d_clock = nullptr;
-    unsigned long long* d_max = nullptr;
+    bool by_size_x = true, by_size_y = true;  // task lengths and CTAs by the size of the batch, not by `tune`
     cudaStream_t stream = nullptr;
     mhd_batch_tuning tune{mhd::kDefaultBatchXRpw, mhd::kDefaultYSeg, 0, 0};
     cudaGraphExec_t graph = nullptr;
-    mhd_batch_tuning graph_tune{};
     long long cells = 0;
 };
 
@@ -72,38 +70,95 @@ const int kTuneXrpw[] = {2, 4, 8, 16};             // x-sweep rows per warp
 const int kTuneYseg[] = {16, 24, 32, 48, 64, 128};  // y-sweep segment rows
 const int kTuneCtasPerSm[] = {2, 3, 4};             // persistent CTAs per SM, both phases
 
-cudaError_t phase(mhd_batch* b, int parity, int which, const mhd_batch_tuning& t, cudaStream_t st) {
-    const int ctas = which == 1 ? t.ctas_x : t.ctas_y;
-    return b->dtype == MHD_F64 ? mhd::launch_batch_f64(b->d_inst, b->d_first, b->n, parity, which, b->solver,
-                                                       b->limiter, t.xrpw, t.yseg, ctas, st)
-                               : mhd::launch_batch_f32(b->d_inst, b->d_first, b->n, parity, which, b->solver,
-                                                       b->limiter, t.xrpw, t.yseg, ctas, st);
+cudaError_t phase(mhd_batch* b, int parity, int which, cudaStream_t st) {
+    const int ctas = which == 1 ? (b->by_size_x ? 0 : b->tune.ctas_x) : which == 2 ? (b->by_size_y ? 0 : b->tune.ctas_y) : 0;
+    const mhd::BatchList& list = b->lists[which > 0 ? which - 1 : 0];
+    return b->dtype == MHD_F64 ? mhd::launch_batch_f64(b->d_inst, list, b->d_ch, b->n, parity, which, b->solver, b->limiter, ctas, st)
+                               : mhd::launch_batch_f32(b->d_inst, list, b->d_ch, b->n, parity, which, b->solver, b->limiter, ctas, st);
 }
 
-// Work decomposition for the current tuning; uploads the table and prefixes.
+// Work lists for the current shape; uploads the tables and drops the graph.
 int build_worklist(mhd_batch* b) {
-    b->first.assign(2 * (b->n + 1), 0);
-    for (int i = 0; i < b->n; ++i) {
-        mhd::BatchInst& I = b->host_inst[i];
-        const int len = mhd::x_seg_len(4 * b->tune.xrpw);
-        I.x_segs = (b->desc[i].nx + len - 1) / len;
-        I.x_pad_ = 0;
-        I.y_strips = (b->desc[i].nx + b->desc[i].ng + 31) / 32;  // strips holding interior columns
-        I.y_bands = (b->desc[i].ny + b->tune.yseg - 1) / b->tune.yseg;
-        I.y_units = (I.y_strips * I.y_bands + mhd::YS_WARPS - 1) / mhd::YS_WARPS;
-        I.pad_ = 0;
-        b->first[i + 1] = b->first[i] + (int)(((long long)I.x_segs * b->desc[i].ny + mhd::BX_WARPS - 1) / mhd::BX_WARPS);
-        b->first[b->n + 1 + i + 1] = b->first[b->n + 1 + i] + I.y_units;
+    const int n = b->n;
+    long long x_work = 0, y_work = 0;
+    for (int i = 0; i < n; ++i) {
+        const mhd_instance_desc& d = b->desc[i];
+        x_work += (long long)d.ny * ((d.nx + 31) / 32);
+        y_work += (long long)d.ny * mhd::y_strips(b->host_inst[i].U);
     }
-    for (int i = 0; i < b->n; ++i) {
-        b->host_inst[b->n + i] = b->host_inst[i];
-        b->host_inst[b->n + i].P.parity = 1;
+    mhd::TaskLen tx{}, ty{};
+    if (b->dtype == MHD_F64) mhd::batch_task_lens_f64(x_work, y_work, tx, ty);
+    else mhd::batch_task_lens_f32(x_work, y_work, tx, ty);
+    static_assert(mhd::BX_WARPS == mhd::YS_WARPS, "a unit is four tasks in both phases");
+    std::vector<mhd::BatchSeg> segs;
+    std::vector<int> units;
+    size_t seg0[4] = {}, unit0[4] = {};
+    for (int l = 0; l < 3; ++l) {
+        for (int i = 0; i < n; ++i) {
+            const int nx = b->desc[i].nx, ny = b->desc[i].ny, strips = mhd::y_strips(b->host_inst[i].U);
+            if (l == 2) {
+                segs.push_back({i, 0, nx * ny, 0, 0, 0, 0, 0, 0});
+                continue;
+            }
+            const bool by_size = l == 0 ? b->by_size_x : b->by_size_y;
+            const mhd::TaskLen& t = l == 0 ? tx : ty;
+            const int cut = by_size && !t.one_wave ? ny - ny / 8 : ny;  // rows from here on in shorter tasks
+            for (int p = 0; p < 2; ++p) {
+                const int r0 = p == 0 ? 0 : cut, r1 = p == 0 ? cut : ny, most = p == 0 ? t.len : (t.len + 2) / 3;
+                if (r0 == r1) continue;
+                if (l == 0) {
+                    int len = mhd::x_seg_len(4 * b->tune.xrpw);
+                    if (by_size) {  // equal segments, the fewest of `most` chunks
+                        const int k = mhd::x_seg_len(most), parts = (nx + k - 1) / k;
+                        len = mhd::x_seg_len(((nx + parts - 1) / parts + 4 + 31) / 32);
+                    }
+                    segs.push_back({i, 0, nx, len, (nx + len - 1) / len, r0, r1 - r0, 0, 0});
+                } else {
+                    int len = b->tune.yseg;
+                    if (by_size) {
+                        const int parts = (r1 - r0 + most - 1) / most;
+                        len = (r1 - r0 + parts - 1) / parts;
+                    }
+                    segs.push_back({i, r0, r1, len, (r1 - r0 + len - 1) / len, 0, strips, 0, 0});
+                }
+            }
+        }
+        const auto begin = segs.begin() + seg0[l];
+        if (l < 2) std::stable_sort(begin, segs.end(), [](const mhd::BatchSeg& p, const mhd::BatchSeg& q) { return p.len > q.len; });
+        std::vector<char> led(n, 0);
+        for (auto s = begin; s != segs.end(); ++s) {
+            const long long count = l < 2 ? ((long long)s->n * s->width + mhd::YS_WARPS - 1) / mhd::YS_WARPS
+                                          : ((long long)s->hi + mhd::kMaxUnit - 1) / mhd::kMaxUnit;
+            s->lead = !led[s->inst];
+            led[s->inst] = 1;
+            s->unit = (int)(units.size() - unit0[l]);
+            if ((long long)s->unit + count > 0x7fffffff) return berr(MHD_ERR_ARG, "batch: too many work units");
+            units.insert(units.end(), (size_t)count, (int)(s - begin));
+        }
+        seg0[l + 1] = segs.size();
+        unit0[l + 1] = units.size();
+    }
+    for (int i = 0; i < n; ++i) {
+        b->host_inst[n + i] = b->host_inst[i];
+        b->host_inst[n + i].P.parity = 1;
+    }
+    if (units.size() > b->units_cap) {
+        if (b->d_units) cudaFree(b->d_units);
+        b->d_units = nullptr;
+        b->units_cap = 0;
+        if (cudaMalloc(&b->d_units, sizeof(int) * units.size()) != cudaSuccess) {
+            b->d_units = nullptr;
+            return berr(MHD_ERR_NOMEM, "batch: work list");
+        }
+        b->units_cap = units.size();
     }
     BCK(cudaMemcpyAsync(b->d_inst, b->host_inst.data(), sizeof(mhd::BatchInst) * b->host_inst.size(),
                         cudaMemcpyHostToDevice, b->stream));
-    BCK(cudaMemcpyAsync(b->d_first, b->first.data(), sizeof(int) * b->first.size(), cudaMemcpyHostToDevice,
-                        b->stream));
+    BCK(cudaMemcpyAsync(b->d_seg, segs.data(), sizeof(mhd::BatchSeg) * segs.size(), cudaMemcpyHostToDevice, b->stream));
+    BCK(cudaMemcpyAsync(b->d_units, units.data(), sizeof(int) * units.size(), cudaMemcpyHostToDevice, b->stream));
     BCK(cudaStreamSynchronize(b->stream));
+    for (int l = 0; l < 3; ++l)
+        b->lists[l] = {b->d_seg + seg0[l], b->d_units + unit0[l], (int)(unit0[l + 1] - unit0[l])};
     if (b->graph) {
         cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;
@@ -113,16 +168,9 @@ int build_worklist(mhd_batch* b) {
 
 // Every clock from its instance's CFL maximum (floored by the carried c_h).
 int start_clocks(mhd_batch* b) {
-    BCK(cudaMemsetAsync(b->d_max, 0, sizeof(unsigned long long) * b->n, b->stream));
-    for (int i = 0; i < b->n; ++i) {
-        mhd::DevGrid g{b->U[i].data, b->U[i].pitch, b->U[i].plane, b->U[i].nx, b->U[i].ny, b->U[i].ng, 0};
-        const cudaError_t e =
-            b->dtype == MHD_F64 ? mhd::launch_max_speed_f64(g, b->desc[i].gamma, b->ch[i], b->d_max + i, b->stream, b->nsm)
-                                : mhd::launch_max_speed_f32(g, b->desc[i].gamma, b->ch[i], b->d_max + i, b->stream, b->nsm);
-        BCK(e);
-    }
-    batch_clock_init<<<(b->n + 127) / 128, 128, 0, b->stream>>>(b->d_clock, b->d_max, b->n);
-    BCK(cudaGetLastError());
+    BCK(cudaMemsetAsync(b->d_clock, 0, sizeof(mhd::DevClock) * b->n, b->stream));  // t = 0, no steps, running
+    BCK(cudaMemcpyAsync(b->d_ch, b->ch.data(), sizeof(double) * b->n, cudaMemcpyHostToDevice, b->stream));
+    BCK(phase(b, 0, 3, b->stream));
     return MHD_OK;
 }
 
@@ -175,9 +223,9 @@ int mhd_batch_create(const mhd_instance_desc* desc, int n, int dtype, int solver
         b->cells += (long long)d.nx * d.ny;
     }
     if (!rc && (cudaMalloc(&b->d_inst, sizeof(mhd::BatchInst) * 2 * n) != cudaSuccess ||
-                cudaMalloc(&b->d_first, sizeof(int) * 2 * (n + 1)) != cudaSuccess ||
-                cudaMalloc(&b->d_clock, sizeof(mhd::DevClock) * n) != cudaSuccess ||
-                cudaMalloc(&b->d_max, sizeof(unsigned long long) * n) != cudaSuccess))
+                cudaMalloc(&b->d_seg, sizeof(mhd::BatchSeg) * 5 * n) != cudaSuccess ||
+                cudaMalloc(&b->d_ch, sizeof(double) * n) != cudaSuccess ||
+                cudaMalloc(&b->d_clock, sizeof(mhd::DevClock) * n) != cudaSuccess))
         rc = berr(MHD_ERR_NOMEM, "mhd_batch_create: device tables");
     if (rc) {
         mhd_batch_destroy(b);
@@ -187,7 +235,7 @@ int mhd_batch_create(const mhd_instance_desc* desc, int n, int dtype, int solver
         const mhd_instance_desc& d = desc[i];
         mhd::BatchInst& I = b->host_inst[i];
         I.U = mhd::DevGrid{b->U[i].data, b->U[i].pitch, b->U[i].plane, d.nx, d.ny, d.ng, 0};
-        I.T = mhd::DevGrid{b->T[i].data, b->T[i].pitch, b->T[i].plane, d.nx, d.ny, d.ng, 0};
+        I.T = b->T[i].data;
         mhd::StepParams& P = I.P;
         std::memset(&P, 0, sizeof P);
         P.gamma = d.gamma;
@@ -220,9 +268,10 @@ int mhd_batch_destroy(mhd_batch* b) {
     for (auto& g : b->U) mhd_grid_free(&g);
     for (auto& g : b->T) mhd_grid_free(&g);
     if (b->d_inst) cudaFree(b->d_inst);
-    if (b->d_first) cudaFree(b->d_first);
+    if (b->d_units) cudaFree(b->d_units);
     if (b->d_clock) cudaFree(b->d_clock);
-    if (b->d_max) cudaFree(b->d_max);
+    if (b->d_seg) cudaFree(b->d_seg);
+    if (b->d_ch) cudaFree(b->d_ch);
     delete b;
     return MHD_OK;
 }
@@ -260,6 +309,7 @@ int mhd_batch_set_tuning(mhd_batch* b, const mhd_batch_tuning* t) {
     if (t->xrpw < 1 || t->xrpw > 64 || t->yseg < 4 || t->yseg > 4096 || t->ctas_x < 0 || t->ctas_y < 0)
         return berr(MHD_ERR_ARG, "mhd_batch_set_tuning: out of range");
     b->tune = *t;
+    b->by_size_x = b->by_size_y = false;
     default_ctas(b);
     return build_worklist(b);
 }
@@ -270,11 +320,7 @@ int mhd_batch_run(mhd_batch* b, int max_steps, mhd_run_info* info) {
     if (max_steps < 1) return berr(MHD_ERR_ARG, "mhd_batch_run: max_steps must be >= 1");
     int rc = start_clocks(b);
     if (rc) return rc;
-    if (!b->graph || std::memcmp(&b->graph_tune, &b->tune, sizeof b->tune) != 0) {
-        if (b->graph) {
-            cudaGraphExecDestroy(b->graph);
-            b->graph = nullptr;
-        }
+    if (!b->graph) {
         cudaStream_t cap = b->stream;
         bool own = false;
         if (!cap) {
@@ -282,12 +328,12 @@ int mhd_batch_run(mhd_batch* b, int max_steps, mhd_run_info* info) {
             own = true;
         }
         cudaGraph_t gr = nullptr;
-        BCK(phase(b, 0, 0, b->tune, cap));  // kernel attribute set-up, outside the capture
+        BCK(phase(b, 0, 0, cap));  // kernel attribute set-up, outside the capture
         BCK(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
         cudaError_t e = cudaSuccess;
         for (int p = 0; p < 2 && e == cudaSuccess; ++p) {
-            e = phase(b, p, 1, b->tune, cap);
-            if (e == cudaSuccess) e = phase(b, p, 2, b->tune, cap);
+            e = phase(b, p, 1, cap);
+            if (e == cudaSuccess) e = phase(b, p, 2, cap);
         }
         const cudaError_t e2 = cudaStreamEndCapture(cap, &gr);
         if (own) cudaStreamDestroy(cap);
@@ -301,12 +347,11 @@ int mhd_batch_run(mhd_batch* b, int max_steps, mhd_run_info* info) {
             b->graph = nullptr;
             return berr(MHD_ERR_CUDA, "mhd_batch_run: graph instantiation failed");
         }
-        b->graph_tune = b->tune;
     }
     for (int p = 0; p < max_steps / 2; ++p) BCK(cudaGraphLaunch(b->graph, b->stream));
     if (max_steps & 1) {
-        BCK(phase(b, 0, 1, b->tune, b->stream));
-        BCK(phase(b, 0, 2, b->tune, b->stream));
+        BCK(phase(b, 0, 1, b->stream));
+        BCK(phase(b, 0, 2, b->stream));
     }
     std::vector<mhd::DevClock> hc(b->n);
     BCK(cudaMemcpyAsync(hc.data(), b->d_clock, sizeof(mhd::DevClock) * b->n, cudaMemcpyDeviceToHost, b->stream));
@@ -362,21 +407,21 @@ int mhd_batch_tune(mhd_batch* b, int reps, mhd_batch_tuning* best_out) {
     const auto& ys = kTuneYseg;
     const auto& yc = kTuneCtasPerSm;
     auto time_phase = [&](int which, float* ms) -> int {
-        BCK(phase(b, 0, which, b->tune, b->stream));  // warm
+        BCK(phase(b, 0, which, b->stream));  // warm
         BCK(cudaEventRecord(e0, b->stream));
-        for (int r = 0; r < reps; ++r) BCK(phase(b, 0, which, b->tune, b->stream));
+        for (int r = 0; r < reps; ++r) BCK(phase(b, 0, which, b->stream));
         BCK(cudaEventRecord(e1, b->stream));
         BCK(cudaEventSynchronize(e1));
         BCK(cudaEventElapsedTime(ms, e0, e1));
         return MHD_OK;
     };
-    float best_ms = 1e30f;
+    float best_ms = 1e30f, ms = 0.f;
+    b->by_size_x = false;
     for (int r : xr)
         for (int c : xc) {
             b->tune.xrpw = r;
             b->tune.ctas_x = c * b->nsm;
             if ((rc = build_worklist(b))) return rc;
-            float ms = 0.f;
             if ((rc = time_phase(1, &ms))) return rc;
             if (ms < best_ms) {
                 best_ms = ms;
@@ -386,15 +431,17 @@ int mhd_batch_tune(mhd_batch* b, int reps, mhd_batch_tuning* best_out) {
         }
     b->tune.xrpw = best.xrpw;
     b->tune.ctas_x = best.ctas_x;
+    b->by_size_x = true;
     if ((rc = build_worklist(b))) return rc;
-    BCK(phase(b, 0, 1, b->tune, b->stream));  // T from U with the chosen x tuning
+    if ((rc = time_phase(1, &ms))) return rc;  // T from U
+    b->by_size_x = ms < best_ms;
     best_ms = 1e30f;
+    b->by_size_y = false;
     for (int s : ys)
         for (int c : yc) {
             b->tune.yseg = s;
             b->tune.ctas_y = c * b->nsm;
             if ((rc = build_worklist(b))) return rc;
-            float ms = 0.f;
             if ((rc = time_phase(2, &ms))) return rc;
             if (ms < best_ms) {
                 best_ms = ms;
@@ -402,6 +449,10 @@ int mhd_batch_tune(mhd_batch* b, int reps, mhd_batch_tuning* best_out) {
                 best.ctas_y = c * b->nsm;
             }
         }
+    b->by_size_y = true;
+    if ((rc = build_worklist(b))) return rc;
+    if ((rc = time_phase(2, &ms))) return rc;
+    b->by_size_y = ms < best_ms;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     b->tune = best;

@@ -60,13 +60,21 @@ cudaError_t launch_step_f32(const DevGrid& in, const DevGrid& tmp, const DevGrid
 // strides not 16-byte multiples) or the driver has no encoder.
 bool rows_tensor_map(void* map64, const DevGrid& g, int elem_bytes, int box_cols, int box_rows);
 
-// Batched instances: one persistent launch per sweep over the global work list
-// (batch.cuh).  which = 1: x-sweeps of every instance, 2: y-sweeps.
+// Batched instances: one launch per sweep over the global work list (batch.cuh).
+// which = 1: x-sweeps of every instance, 2: y-sweeps, 3: the CFL maximum of every
+// instance (floored by ch[i]) into slot 0 of its clock, 0: the one-time kernel
+// attribute setup.  ctas: CTAs striding over the list (0: one per unit).
 struct BatchInst;
-cudaError_t launch_batch_f64(const BatchInst* inst, const int* first, int n, int parity, int which, int solver,
-                             int limiter, int xrpw, int yseg, int ctas, cudaStream_t st);
-cudaError_t launch_batch_f32(const BatchInst* inst, const int* first, int n, int parity, int which, int solver,
-                             int limiter, int xrpw, int yseg, int ctas, cudaStream_t st);
+struct BatchList;
+struct TaskLen;
+cudaError_t launch_batch_f64(const BatchInst* inst, const BatchList& list, const double* ch, int n, int parity, int which,
+                             int solver, int limiter, int ctas, cudaStream_t st);
+cudaError_t launch_batch_f32(const BatchInst* inst, const BatchList& list, const double* ch, int n, int parity, int which,
+                             int solver, int limiter, int ctas, cudaStream_t st);
+// Longest x and y tasks by the size of the batch (x: 32-cell chunks of all
+// instances' rows, y: rows of all instances' strips).
+void batch_task_lens_f64(long long x_work, long long y_work, TaskLen& x, TaskLen& y);
+void batch_task_lens_f32(long long x_work, long long y_work, TaskLen& x, TaskLen& y);
 
 // riemann_flux of n faces (AoS, 9 doubles per face, device memory) with the
 // precision's own solver functions; dir 0 = x, 1 = y.

@@ -99,9 +99,13 @@ cudaError_t launch_step_f32(const DevGrid& in, const DevGrid& tmp, const DevGrid
     return dispatch_step<FastPolicy>(in, tmp, out, P, st, yseg, which, xrpw, ystage);
 }
 
-cudaError_t launch_batch_f32(const BatchInst* inst, const int* first, int n, int parity, int which, int solver,
-                             int limiter, int xrpw, int yseg, int ctas, cudaStream_t st) {
-    return dispatch_batch<FastPolicy>(inst, first, n, parity, which, solver, limiter, xrpw, yseg, ctas, st);
+cudaError_t launch_batch_f32(const BatchInst* inst, const BatchList& list, const double* ch, int n, int parity, int which,
+                             int solver, int limiter, int ctas, cudaStream_t st) {
+    return dispatch_batch<FastPolicy>(inst, list, ch, n, parity, which, solver, limiter, ctas, st);
+}
+
+void batch_task_lens_f32(long long x_work, long long y_work, TaskLen& x, TaskLen& y) {
+    batch_task_lens<FastPolicy<HLL, MINMOD>>(x_work, y_work, x, y);
 }
 
 cudaError_t launch_faces_f32(const double* UL, const double* UR, long long n, int dir, int solver, double ch,
