@@ -54,23 +54,6 @@ ADJ_HD Pr<double> nmad(const Pr<double>& a, const Pr<double>& b, const Pr<double
 template <typename R>
 ADJ_HD Pr<R> operator*(R a, const Pr<R>& b) { return dup(a) * b; }
 
-// 1 / a.  FP64 on the device: the hardware's first approximation (20 bits) and
-// one third-order step, y (1 + e + e^2) with e = 1 - a y, which leaves the error
-// of its own roundings (under 2 ulp); no branch, so the chains of a cell's many
-// reciprocals interleave, which the divide's branches prevent.  Zeros,
-// infinities and NaN give NaN, which the positivity tests treat as they treat
-// the infinities of a divide.
-ADJ_HD float rcp(float a) { return 1.0f / a; }
-ADJ_HD double rcp(double a) {
-#ifdef __CUDA_ARCH__
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-    const double e = fma(-a, y, 1.0);
-    return fma(y, fma(e, e, e), y);
-#else
-    return 1.0 / a;
-#endif
-}
 // Correctly rounded, whatever the translation unit's flags.
 ADJ_HD float rcp_rn(float a) {
 #ifdef __CUDA_ARCH__
@@ -313,7 +296,7 @@ ADJ_HD void root(float x, float& s, float& is) {
 #endif
 }
 ADJ_HD void root(double x, double& s, double& is) {
-    s = sqrt(x > 0.0 ? x : 0.0);
+    s = x > 0.0 ? sqrt_of(x) : 0.0;
     is = x > 0.0 ? rcp(s) : 0.0;
 }
 
@@ -400,8 +383,8 @@ ADJ_HD void hlld_pair(const Pr<R>* U, R ch, R g, R dtd, const R* d, Pr<R>* lU, R
     R UL[NV], UR[NV], f[NV], lF[NV], lL[NV], lR[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k) { UL[k] = U[k].x; UR[k] = U[k].y; lF[k] = dtd * d[k]; lL[k] = lR[k] = R(0); }
-    face<HLLD>(UL, UR, ch, g, f);
-    face_adj<HLLD>(UL, UR, ch, g, lF, lL, lR, lch);
+    const bool fine = hlld_face(UL, UR, ch, g, f);
+    hlld_face_adj(UL, UR, ch, g, fine, lF, lL, lR, lch);
 #pragma unroll
     for (int k = 0; k < NV; ++k) { ldtd += f[k] * d[k]; lU[k] = {lL[k], lR[k]}; }
 }

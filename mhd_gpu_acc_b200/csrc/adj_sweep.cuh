@@ -19,7 +19,8 @@ namespace mhd {
 namespace adj {
 
 constexpr int AT = 26;      // outputs per warp: 32 lanes minus a 3-cell halo on each side
-constexpr int AWARPS = 8;   // warps per CTA; columns of a y block
+constexpr int AWARPS = 8;   // warps per y CTA: the columns of its block
+constexpr int AXWARPS = 4;  // warps per x CTA
 constexpr int APITCH = AWARPS + 1;
 
 template <typename R>
@@ -93,6 +94,10 @@ __device__ __forceinline__ void adj_cell(const R* Uc, const R* lT, int p, int lo
     zero(lWm);
     zero(lWc);
     zero(lWp);
+    // the neighbours' W again (18 shuffles) rather than held across the face, which
+    // needs the registers
+    shfl_up_n<NV>(W, Wm, 1);
+    shfl_down_n<NV>(W, Wp, 1);
     if (do_recon) {
         R sd = R(0), sc = R(0);
         recon_adj2<LIM>(Wm, W, Wp, rc, dtd, ch, igm1, gr, lS, lWm, lWc, lWp, sd, sc);
@@ -116,10 +121,10 @@ __device__ __forceinline__ void adj_cell(const R* Uc, const R* lT, int p, int lo
     lU[PSI] += lWc[PSI];
 }
 
-// Sums of a CTA into acc[0..N): one atomic per value and CTA.
-template <int N>
+// Sums of a CTA of WARPS warps into acc[0..N): one atomic per value and CTA.
+template <int N, int WARPS>
 __device__ __forceinline__ void block_add(const double* v, double* acc) {
-    __shared__ double part[N][AWARPS];
+    __shared__ double part[N][WARPS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int q = 0; q < N; ++q) {
@@ -132,17 +137,17 @@ __device__ __forceinline__ void block_add(const double* v, double* acc) {
     if (threadIdx.x < N) {
         double s = 0.0;
 #pragma unroll
-        for (int w = 0; w < AWARPS; ++w) s += part[threadIdx.x][w];
+        for (int w = 0; w < WARPS; ++w) s += part[threadIdx.x][w];
         if (s != 0.0) atomicAdd(acc + threadIdx.x, s);
     }
 }
 
 // x: rows, one tile of a row per warp; lamOut's ghost rows folded on read.
 template <typename R, int LIM, int SOLVER>
-__global__ void __launch_bounds__(32 * AWARPS, AdjShape<R, SOLVER>::kBlocks)
+__global__ void __launch_bounds__(32 * AXWARPS, AdjShape<R, SOLVER>::kXBlocks)
     adj_x_kernel(DevGrid U, DevGrid lamOut, DevGrid lamIn, R g, R gm1, R igm1, R dtd, R ch, double* acc) {
     const int lane = threadIdx.x & 31;
-    const long long warp = (long long)blockIdx.x * AWARPS + (threadIdx.x >> 5);
+    const long long warp = (long long)blockIdx.x * AXWARPS + (threadIdx.x >> 5);
     const int ng = U.ng, lo = ng, hi = ng + U.nx;
     const int ntile = (U.nx + 4 + AT - 1) / AT;
     const int row = (int)(warp / ntile), tile = (int)(warp - (long long)row * ntile);
@@ -163,14 +168,14 @@ __global__ void __launch_bounds__(32 * AWARPS, AdjShape<R, SOLVER>::kBlocks)
         if (own && p >= lo - 2 && p < hi + 2) store_cell(lamIn, p, j, lU);
     }
     const double v[2] = {(double)ldtd, (double)lch};
-    block_add<2>(v, acc);
+    block_add<2, AXWARPS>(v, acc);
 }
 
 // y: columns, eight per CTA; lamOut's ghost columns folded and its interior psi
 // cotangent scaled by the damping factor f on read, sum(lambda_psi psi_next / f)
 // to acc[2].
 template <typename R, int LIM, int SOLVER>
-__global__ void __launch_bounds__(32 * AWARPS, AdjShape<R, SOLVER>::kBlocks)
+__global__ void __launch_bounds__(32 * AWARPS, AdjShape<R, SOLVER>::kYBlocks)
     adj_y_kernel(DevGrid U, DevGrid lamOut, DevGrid lamIn, DevGrid Unext, R g, R gm1, R igm1, R dtd, R ch, double f,
                  double* acc) {
     extern __shared__ __align__(16) unsigned char ay_smem[];
@@ -233,7 +238,7 @@ __global__ void __launch_bounds__(32 * AWARPS, AdjShape<R, SOLVER>::kBlocks)
         }
     }
     const double v[3] = {(double)ldtd, (double)lch, sf};
-    block_add<3>(v, acc);
+    block_add<3, AWARPS>(v, acc);
 }
 
 template <typename R, int LIM, int SOLVER>
@@ -241,7 +246,7 @@ cudaError_t launch_one(const AdjSweepArgs& a, cudaStream_t st) {
     const R g = (R)a.gamma, gm1 = (R)(a.gamma - 1.0), igm1 = (R)(1.0 / (a.gamma - 1.0));
     if (a.dir == 0) {
         const long long warps = (long long)a.U.ny * ((a.U.nx + 4 + AT - 1) / AT);
-        adj_x_kernel<R, LIM, SOLVER><<<(unsigned)((warps + AWARPS - 1) / AWARPS), 32 * AWARPS, 0, st>>>(
+        adj_x_kernel<R, LIM, SOLVER><<<(unsigned)((warps + AXWARPS - 1) / AXWARPS), 32 * AXWARPS, 0, st>>>(
             a.U, a.lamOut, a.lamIn, g, gm1, igm1, (R)a.dtd, (R)a.ch, a.acc);
     } else {
         constexpr int bytes = 2 * NV * 32 * APITCH * (int)sizeof(R);
