@@ -93,20 +93,29 @@ __global__ void speed_adj_kernel(DevGrid U, DevGrid lam, const int* idx_p, R g, 
 // Called for a step n1 whose own maximum set c_h, with the steps n1 .. n2 not
 // yet combined: a step n > n1 passes its weight on as the floor of step n - 1
 // and step n1's argmax cell takes *lm.  Explicit round-to-nearest operations.
-__global__ void step_scalars_kernel(const double* sc, const double* log, int n1, int n2, double cr, double dx,
-                                    double dy, double* lm, int* idx) {
+// One warp: the terms of 32 steps at once, then their chain in step order (a
+// one-thread loop waited for memory at every step: 22 -> 4 us for 30 steps).
+__global__ void __launch_bounds__(32) step_scalars_kernel(const double* sc, const double* log, int n1, int n2, double cr,
+                                                         double dx, double dy, double* lm, int* idx) {
     double carry = 0.0;
-    for (int n = n2; n >= n1; --n) {
-        const double* s = sc + 5 * n;
-        const double dt = log[3 * n], ch = log[3 * n + 1], f = log[3 * n + 2];
-        const double ldt = __dadd_rn(__dadd_rn(__ddiv_rn(s[3], dx), __ddiv_rn(s[0], dy)),
-                                     __dmul_rn(__dmul_rn(s[2], f), __ddiv_rn(-ch, cr)));
-        const double lch = __dadd_rn(__dadd_rn(__dadd_rn(s[4], s[1]), __dmul_rn(__dmul_rn(s[2], f), __ddiv_rn(-dt, cr))),
-                                     carry);
-        carry = __dadd_rn(lch, __dmul_rn(ldt, __ddiv_rn(-dt, ch)));
+    for (int top = n2; top >= n1; top -= 32) {
+        const int n = top - (int)threadIdx.x;
+        double own = 0.0, slope = 0.0;
+        if (n >= n1) {
+            const double* s = sc + 5 * n;
+            const double dt = log[3 * n], ch = log[3 * n + 1], f = log[3 * n + 2];
+            const double ldt = __dadd_rn(__dadd_rn(__ddiv_rn(s[3], dx), __ddiv_rn(s[0], dy)),
+                                         __dmul_rn(__dmul_rn(s[2], f), __ddiv_rn(-ch, cr)));
+            own = __dadd_rn(__dadd_rn(s[4], s[1]), __dmul_rn(__dmul_rn(s[2], f), __ddiv_rn(-dt, cr)));
+            slope = __dmul_rn(ldt, __ddiv_rn(-dt, ch));
+        }
+        for (int k = 0; k < 32 && top - k >= n1; ++k)
+            carry = __dadd_rn(__dadd_rn(__shfl_sync(FULL, own, k), carry), __shfl_sync(FULL, slope, k));
     }
-    *lm = carry;
-    *idx = INT_MAX;
+    if (threadIdx.x == 0) {
+        *lm = carry;
+        *idx = INT_MAX;
+    }
 }
 
 // grad_k += sum over every cell (ghosts included) of lambda_0 . dU0/da_k for the
@@ -188,6 +197,7 @@ struct mhd_adjoint {
     mhd_workspace* ws = nullptr;
     double* d_target = nullptr;          // ny * nx
     mhd::DevClock* d_clock = nullptr;    // of the forward solve
+    unsigned long long* d_acc = nullptr;  // the CFL maximum's scratch (MaxOut), zero between launches
     double* d_log = nullptr;             // {dt, ch, damp} of each step, then J: one block that the host reads once
     double* d_sc = nullptr;              // 5 reverse sums per step, then the argmax weight
     double* d_grad = nullptr;            // 16
@@ -274,11 +284,13 @@ int forward(mhd_adjoint* a, const double* amp, double* J, double* rho_final, con
     ACK(cudaMemsetAsync(a->d_log, 0, sizeof(double) * a->log_len(), st));
     ARC(mhd_initialise_orszag_tang(a->ws, &a->seg[0], a->b0, a->gamma, amp));
     if (!a->ckpt.empty()) ARC(grid_copy(a->ckpt[0], a->seg[0], st));
-    mhd::DevClock clock{};
-    clock.log = a->d_log;
-    ACK(cudaMemcpyAsync(a->d_clock, &clock, sizeof clock, cudaMemcpyHostToDevice, st));
-    ACK(f64(a) ? mhd::launch_max_speed_f64(dg(a->seg[0]), a->gamma, 0.0, &a->d_clock->maxbits[0], st, mhd::kSMs)
-               : mhd::launch_max_speed_f32(dg(a->seg[0]), a->gamma, 0.0, &a->d_clock->maxbits[0], st, mhd::kSMs));
+    mhd::MaxOut out{};
+    out.acc = a->d_acc;
+    out.count = reinterpret_cast<unsigned*>(a->d_acc + 1);
+    out.clock = a->d_clock;
+    out.log = a->d_log;
+    ACK(f64(a) ? mhd::launch_max_speed_f64(dg(a->seg[0]), a->gamma, 0.0, out, st)
+               : mhd::launch_max_speed_f32(dg(a->seg[0]), a->gamma, 0.0, out, st));
     int last = 0;
     for (int n = 0; n < a->nsteps; ++n) {
         const int i = n % a->every;
@@ -340,7 +352,7 @@ int reverse_step(mhd_adjoint* a, int n, int i, const mhd_grid& lam_next, const m
     const double ch_prev = n > 0 ? a->log[3 * n - 2] : 0.0;
     if (ch > ch_prev) {
         double* lm = a->d_sc + 5 * a->nsteps;
-        mhd::adj::step_scalars_kernel<<<1, 1, 0, st>>>(a->d_sc, a->d_log, n, *pending, a->cr, dx, dy, lm, a->d_idx);
+        mhd::adj::step_scalars_kernel<<<1, 32, 0, st>>>(a->d_sc, a->d_log, n, *pending, a->cr, dx, dy, lm, a->d_idx);
         ACK(cudaGetLastError());
         ACK(f64(a) ? mhd::launch_argmax_f64(dg(a->seg[i]), a->gamma, ch_prev, ch, a->d_idx, st)
                    : mhd::launch_argmax_f32(dg(a->seg[i]), a->gamma, ch_prev, ch, a->d_idx, st));
@@ -440,6 +452,8 @@ int mhd_adjoint_create(int nx, int ny, int dtype, int limiter, double gamma, dou
     if (!rc) rc = mhd_set_cr(a->ws, cr);
     if (!rc && (cudaMalloc(&a->d_target, sizeof(double) * (size_t)nx * ny) != cudaSuccess ||
                 cudaMalloc(&a->d_clock, sizeof(mhd::DevClock)) != cudaSuccess ||
+                cudaMalloc(&a->d_acc, 2 * sizeof(unsigned long long)) != cudaSuccess ||
+                cudaMemset(a->d_acc, 0, 2 * sizeof(unsigned long long)) != cudaSuccess ||
                 cudaMalloc(&a->d_log, sizeof(double) * a->log_len()) != cudaSuccess ||
                 cudaMalloc(&a->d_grad, sizeof(double) * 16) != cudaSuccess ||
                 cudaMalloc(&a->d_idx, sizeof(int)) != cudaSuccess ||
@@ -467,6 +481,7 @@ int mhd_adjoint_destroy(mhd_adjoint* a) {
     if (a->ws) mhd_workspace_destroy(a->ws);
     if (a->d_target) cudaFree(a->d_target);
     if (a->d_clock) cudaFree(a->d_clock);
+    if (a->d_acc) cudaFree(a->d_acc);
     if (a->d_log) cudaFree(a->d_log);
     if (a->d_grad) cudaFree(a->d_grad);
     if (a->d_idx) cudaFree(a->d_idx);

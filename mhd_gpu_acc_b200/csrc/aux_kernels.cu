@@ -183,20 +183,6 @@ __global__ void __launch_bounds__(DIAG_THREADS) diag_final_kernel(const double* 
     }
 }
 
-__global__ void clock_init_kernel(DevClock* c, const unsigned long long* max0) {
-    c->maxbits[0] = *max0;
-    c->maxbits[1] = 0ull;
-    c->t[0] = 0.0;
-    c->t[1] = 0.0;
-    c->last_dt = 0.0;
-    c->last_ch = 0.0;
-    c->steps = 0;
-    c->status = CLK_OK;
-    c->lowbeta_hits = 0u;
-    c->flux_fallbacks = 0u;
-    c->log = nullptr;
-}
-
 unsigned grid_for(long long n, int threads) {
     long long b = (n + threads - 1) / threads;
     if (b > 65535LL * 4) b = 65535LL * 4;
@@ -248,11 +234,6 @@ cudaError_t launch_diagnostics(const DevGrid& g, int elem_bytes, double gamma, d
     else
         diag_partial_kernel<float><<<DIAG_BLOCKS, DIAG_THREADS, 0, st>>>(g, gamma, dx, dy, scratch);
     diag_final_kernel<<<1, DIAG_THREADS, 0, st>>>(scratch, dx * dy, out);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_clock_init(DevClock* c, const unsigned long long* max0, cudaStream_t st) {
-    clock_init_kernel<<<1, 1, 0, st>>>(c, max0);
     return cudaGetLastError();
 }
 

@@ -8,6 +8,7 @@
 #include <atomic>
 #include <cfloat>
 #include <cstdarg>
+#include <cstddef>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -108,10 +109,20 @@ struct mhd_workspace {
     double dx = 0.0, dy = 0.0;     // cell spacing of the step; 0 = from the grid's extent
     int nsm = 148;
     cudaStream_t stream = nullptr;
-    unsigned long long* d_max = nullptr;
-    mhd::DevClock* d_clock = nullptr;
-    int* d_fault = nullptr;       // ClockStatus bits from bounded device waits
-    double* d_diag = nullptr;     // 6 * 1024 partials + 6 results
+    struct Device {               // device scratch, one allocation
+        mhd::DevClock clock;
+        int fault;                // ClockStatus bits from bounded device waits (behind the clock: one copy reads both)
+        unsigned max_count;       // the CFL maximum's scratch, zero between launches
+        unsigned long long max_acc;
+        double diag[6 * 1024 + 8];  // 6 * 1024 partials + 6 results
+    };
+    struct Host {                 // page-locked: what the device hands back
+        mhd::DevClock clock;
+        int fault;
+        unsigned long long max[2];  // CFL maximum bits, fault word
+    };
+    Device* d = nullptr;
+    Host* h = nullptr;
     void* d_stage = nullptr;      // FP64 staging for uploads/downloads
     size_t stage_bytes = 0;
     // graph of two captured steps
@@ -125,16 +136,27 @@ struct mhd_workspace {
 
 namespace {
 
-// Reads (and clears) the fault word after the stream has drained: a bounded
-// device wait that gave up turns into MHD_ERR_TIMEOUT.
+// A fault word read back: a bounded device wait that gave up turns into
+// MHD_ERR_TIMEOUT (and the word is cleared).
+int fault_code(mhd_workspace* ws, int f, const char* what) {
+    if (f == 0) return MHD_OK;
+    cudaMemsetAsync(&ws->d->fault, 0, sizeof(int), ws->stream);
+    return fail(MHD_ERR_TIMEOUT, "%s: a bounded wait for a staged tile gave up (status %d)", what, f);
+}
+
+// Reads (and clears) the fault word after the stream has drained.
 int check_fault(mhd_workspace* ws, const char* what) {
-    int f = 0;
-    if (cudaMemcpyAsync(&f, ws->d_fault, sizeof f, cudaMemcpyDeviceToHost, ws->stream) != cudaSuccess ||
+    if (cudaMemcpyAsync(&ws->h->fault, &ws->d->fault, sizeof(int), cudaMemcpyDeviceToHost, ws->stream) != cudaSuccess ||
         cudaStreamSynchronize(ws->stream) != cudaSuccess)
         return fail(MHD_ERR_CUDA, "%s: %s", what, cudaGetErrorString(cudaGetLastError()));
-    if (f == 0) return MHD_OK;
-    cudaMemsetAsync(ws->d_fault, 0, sizeof(int), ws->stream);
-    return fail(MHD_ERR_TIMEOUT, "%s: a bounded wait for a staged tile gave up (status %d)", what, f);
+    return fault_code(ws, ws->h->fault, what);
+}
+
+// The clock and the fault word into ws->h, in one copy, after the stream has drained.
+int read_clock(mhd_workspace* ws) {
+    CK(cudaMemcpyAsync(ws->h, ws->d, offsetof(mhd_workspace::Device, fault) + sizeof(int), cudaMemcpyDeviceToHost, ws->stream));
+    CK(cudaStreamSynchronize(ws->stream));
+    return MHD_OK;
 }
 
 int ensure_stage(mhd_workspace* ws, size_t bytes) {
@@ -169,7 +191,7 @@ mhd::StepParams base_params(const mhd_workspace* ws, const mhd_grid* g, int solv
     for (int k = 0; k < 4; ++k) P.bc[k] = bc[k];
     P.any_dirichlet = (bc[0] == MHD_BC_DIRICHLET || bc[1] == MHD_BC_DIRICHLET || bc[2] == MHD_BC_DIRICHLET ||
                        bc[3] == MHD_BC_DIRICHLET);
-    P.fault = ws->d_fault;
+    P.fault = &ws->d->fault;
     P.tma_wait_ns = ws->tma_wait_ns;
     return P;
 }
@@ -182,10 +204,26 @@ cudaError_t launch_step(const mhd_grid* g, const mhd::DevGrid& in, const mhd::De
                                : mhd::launch_step_f32(in, tmp, out, P, st, yseg, which, xrpw, ystage);
 }
 
-cudaError_t launch_max(const mhd_workspace* ws, const mhd_grid* g, cudaStream_t st) {
+// CFL maximum of g: into a fresh device clock, or (to_host) into ws->h->max.
+cudaError_t launch_max(const mhd_workspace* ws, const mhd_grid* g, bool to_host) {
     g_launches += 1;
-    return g->dtype == MHD_F64 ? mhd::launch_max_speed_f64(dev(g), ws->gamma, ws->ch, ws->d_max, st, ws->nsm)
-                               : mhd::launch_max_speed_f32(dev(g), ws->gamma, ws->ch, ws->d_max, st, ws->nsm);
+    mhd::MaxOut out{};
+    out.acc = &ws->d->max_acc;
+    out.count = &ws->d->max_count;
+    out.fault = &ws->d->fault;
+    if (to_host) out.host = ws->h->max;
+    else out.clock = &ws->d->clock;
+    return g->dtype == MHD_F64 ? mhd::launch_max_speed_f64(dev(g), ws->gamma, ws->ch, out, ws->stream)
+                               : mhd::launch_max_speed_f32(dev(g), ws->gamma, ws->ch, out, ws->stream);
+}
+
+// CFL maximum of g on the host.
+int max_on_host(mhd_workspace* ws, const mhd_grid* g, const char* what, double* mx) {
+    CK(launch_max(ws, g, true));
+    CK(cudaStreamSynchronize(ws->stream));
+    const int rc = fault_code(ws, (int)ws->h->max[1], what);
+    std::memcpy(mx, &ws->h->max[0], sizeof *mx);
+    return rc;
 }
 
 int status_code(int s) {
@@ -365,15 +403,12 @@ int mhd_workspace_create(const mhd_grid* g, mhd_workspace** out) {
     cudaGetDevice(&dev_id);
     cudaDeviceGetAttribute(&ws->nsm, cudaDevAttrMultiProcessorCount, dev_id);
     if (ws->nsm <= 0) ws->nsm = 148;
-    if (cudaMalloc(&ws->d_max, sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMalloc(&ws->d_clock, sizeof(mhd::DevClock)) != cudaSuccess ||
-        cudaMalloc(&ws->d_fault, sizeof(int)) != cudaSuccess ||
-        cudaMalloc(&ws->d_diag, sizeof(double) * (6 * 1024 + 8)) != cudaSuccess) {
+    if (cudaMalloc(&ws->d, sizeof(mhd_workspace::Device)) != cudaSuccess ||
+        cudaHostAlloc(&ws->h, sizeof(mhd_workspace::Host), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
         mhd_workspace_destroy(ws);
         return fail(MHD_ERR_NOMEM, "mhd_workspace_create: device scratch");
     }
-    cudaMemset(ws->d_clock, 0, sizeof(mhd::DevClock));
-    cudaMemset(ws->d_fault, 0, sizeof(int));
+    cudaMemset(ws->d, 0, offsetof(mhd_workspace::Device, diag));
     *out = ws;
     return MHD_OK;
 }
@@ -381,10 +416,8 @@ int mhd_workspace_create(const mhd_grid* g, mhd_workspace** out) {
 int mhd_workspace_destroy(mhd_workspace* ws) {
     if (!ws) return MHD_OK;
     if (ws->graph) cudaGraphExecDestroy(ws->graph);
-    if (ws->d_max) cudaFree(ws->d_max);
-    if (ws->d_clock) cudaFree(ws->d_clock);
-    if (ws->d_fault) cudaFree(ws->d_fault);
-    if (ws->d_diag) cudaFree(ws->d_diag);
+    if (ws->d) cudaFree(ws->d);
+    if (ws->h) cudaFreeHost(ws->h);
     if (ws->d_stage) cudaFree(ws->d_stage);
     delete ws;
     return MHD_OK;
@@ -464,14 +497,9 @@ int mhd_compute_dt(mhd_workspace* ws, const mhd_grid* g, double cfl, double* dt)
     int rc = check_ws_grid(ws, g, "mhd_compute_dt");
     if (rc) return rc;
     if (!dt) return fail(MHD_ERR_ARG, "mhd_compute_dt: null dt");
-    CK(cudaMemsetAsync(ws->d_max, 0, sizeof(unsigned long long), ws->stream));
-    CK(launch_max(ws, g, ws->stream));
-    unsigned long long bits = 0;
-    CK(cudaMemcpyAsync(&bits, ws->d_max, sizeof bits, cudaMemcpyDeviceToHost, ws->stream));
-    rc = check_fault(ws, "mhd_compute_dt");  // synchronises the stream
+    double mx = 0.0;
+    rc = max_on_host(ws, g, "mhd_compute_dt", &mx);
     if (rc) return rc;
-    double mx;
-    std::memcpy(&mx, &bits, sizeof mx);
     if (!(mx > 0.0)) {
         *dt = DBL_MAX;
         return fail(MHD_ERR_NO_SPEED, "mhd_compute_dt: non-positive maximum wave speed");
@@ -531,13 +559,8 @@ int mhd_max_speed(mhd_workspace* ws, const mhd_grid* g, double* vmax) {
     int rc = check_ws_grid(ws, g, "mhd_max_speed");
     if (rc) return rc;
     if (!vmax) return fail(MHD_ERR_ARG, "mhd_max_speed: null output");
-    CK(cudaMemsetAsync(ws->d_max, 0, sizeof(unsigned long long), ws->stream));
-    CK(launch_max(ws, g, ws->stream));
-    unsigned long long bits = 0;
-    CK(cudaMemcpyAsync(&bits, ws->d_max, sizeof bits, cudaMemcpyDeviceToHost, ws->stream));
-    rc = check_fault(ws, "mhd_max_speed");  // synchronises the stream
+    rc = max_on_host(ws, g, "mhd_max_speed", vmax);
     if (rc) return rc;
-    std::memcpy(vmax, &bits, sizeof *vmax);
     if (!(*vmax > 0.0)) return fail(MHD_ERR_NO_SPEED, "mhd_max_speed: non-positive maximum wave speed");
     return MHD_OK;
 }
@@ -601,15 +624,12 @@ static int start_device_loop(mhd_workspace* ws, mhd_grid* U, mhd_grid* T, double
     if (U->data == T->data) return fail(MHD_ERR_ARG, "%s: U and T must be distinct", what);
     if (!(t_end > 0.0) || !std::isfinite(t_end) || !(cfl > 0.0))
         return fail(MHD_ERR_ARG, "%s: need finite t_end > 0 and cfl > 0", what);
-    CK(cudaMemsetAsync(ws->d_max, 0, sizeof(unsigned long long), ws->stream));
-    CK(launch_max(ws, U, ws->stream));
-    g_launches += 1;
-    CK(mhd::launch_clock_init(ws->d_clock, ws->d_max, ws->stream));
+    CK(launch_max(ws, U, false));
     *P = base_params(ws, U, solver, bc);
     P->cfl = cfl;
     P->t_end = t_end;
     P->dt_min = 1.0e-8 * t_end;
-    P->clock = ws->d_clock;
+    P->clock = &ws->d->clock;
     P->accumulate = 1;
     return MHD_OK;
 }
@@ -619,10 +639,7 @@ int mhd_clock_start(mhd_workspace* ws, const mhd_grid* U, double cfl, double t_e
     if (rc) return rc;
     if (!(t_end > 0.0) || !std::isfinite(t_end) || !(cfl > 0.0))
         return fail(MHD_ERR_ARG, "mhd_clock_start: need finite t_end > 0 and cfl > 0");
-    CK(cudaMemsetAsync(ws->d_max, 0, sizeof(unsigned long long), ws->stream));
-    CK(launch_max(ws, U, ws->stream));
-    g_launches += 1;
-    CK(mhd::launch_clock_init(ws->d_clock, ws->d_max, ws->stream));
+    CK(launch_max(ws, U, false));
     ws->clk_cfl = cfl;
     ws->clk_t_end = t_end;
     ws->clk_started = 1;
@@ -630,9 +647,9 @@ int mhd_clock_start(mhd_workspace* ws, const mhd_grid* U, double cfl, double t_e
 }
 
 int mhd_clock_slot(mhd_workspace* ws, int parity, void** dptr) {
-    if (!ws || !ws->d_clock) return fail(MHD_ERR_STATE, "mhd_clock_slot: null workspace");
+    if (!ws || !ws->d) return fail(MHD_ERR_STATE, "mhd_clock_slot: null workspace");
     if (!dptr || (parity != 0 && parity != 1)) return fail(MHD_ERR_ARG, "mhd_clock_slot: need parity 0 or 1");
-    *dptr = &ws->d_clock->maxbits[parity];
+    *dptr = &ws->d->clock.maxbits[parity];
     return MHD_OK;
 }
 
@@ -656,7 +673,7 @@ int mhd_sweep_clocked(mhd_workspace* ws, const mhd_grid* in, mhd_grid* out, int 
     P.cfl = ws->clk_cfl;
     P.t_end = ws->clk_t_end;
     P.dt_min = 1.0e-8 * ws->clk_t_end;
-    P.clock = ws->d_clock;
+    P.clock = &ws->d->clock;
     P.accumulate = 1;
     P.parity = parity;
     P.row0 = row0;
@@ -669,10 +686,10 @@ int mhd_sweep_clocked(mhd_workspace* ws, const mhd_grid* in, mhd_grid* out, int 
 }
 
 int mhd_clock_read(mhd_workspace* ws, mhd_run_info* info) {
-    if (!ws || !ws->d_clock) return fail(MHD_ERR_STATE, "mhd_clock_read: null workspace");
-    mhd::DevClock hc;
-    CK(cudaMemcpyAsync(&hc, ws->d_clock, sizeof hc, cudaMemcpyDeviceToHost, ws->stream));
-    CK(cudaStreamSynchronize(ws->stream));
+    if (!ws || !ws->d) return fail(MHD_ERR_STATE, "mhd_clock_read: null workspace");
+    const int crc = read_clock(ws);
+    if (crc) return crc;
+    const mhd::DevClock& hc = ws->h->clock;
     if (hc.steps > 0) ws->ch = hc.last_ch;
     if (info) {
         info->t = hc.t[hc.steps & 1];
@@ -683,7 +700,7 @@ int mhd_clock_read(mhd_workspace* ws, mhd_run_info* info) {
         info->fallbacks = hc.flux_fallbacks;
         info->pad_ = 0;
     }
-    return check_fault(ws, "mhd_clock_read");
+    return fault_code(ws, ws->h->fault, "mhd_clock_read");
 }
 
 int mhd_profile_sweeps(mhd_workspace* ws, mhd_grid* U, mhd_grid* T, double cfl, double t_end, int solver,
@@ -765,8 +782,7 @@ int mhd_run(mhd_workspace* ws, mhd_grid* U, mhd_grid* T, double cfl, double t_en
         ws->key = key;
     }
 
-    mhd::DevClock hc;
-    std::memset(&hc, 0, sizeof hc);
+    const mhd::DevClock& hc = ws->h->clock;
     if (max_steps > 0) {
         for (int p = 0; p < max_steps / 2; ++p) {
             g_launches += 4;
@@ -777,8 +793,7 @@ int mhd_run(mhd_workspace* ws, mhd_grid* U, mhd_grid* T, double cfl, double t_en
             Q.parity = 0;
             CK(launch_step(U, dU, dT, dU, Q, st, ws->yseg, 3, ws->xrpw, ws->ystage));
         }
-        CK(cudaMemcpyAsync(&hc, ws->d_clock, sizeof hc, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
+        if ((rc = read_clock(ws))) return rc;
     } else {
         const int chunk = 32;  // graph launches (64 steps) between host checks
         for (;;) {
@@ -786,8 +801,7 @@ int mhd_run(mhd_workspace* ws, mhd_grid* U, mhd_grid* T, double cfl, double t_en
                 g_launches += 4;
                 CK(cudaGraphLaunch(ws->graph, st));
             }
-            CK(cudaMemcpyAsync(&hc, ws->d_clock, sizeof hc, cudaMemcpyDeviceToHost, st));
-            CK(cudaStreamSynchronize(st));
+            if ((rc = read_clock(ws))) return rc;
             if (hc.status != mhd::CLK_OK) break;
         }
     }
@@ -801,7 +815,7 @@ int mhd_run(mhd_workspace* ws, mhd_grid* U, mhd_grid* T, double cfl, double t_en
         info->fallbacks = hc.flux_fallbacks;
         info->pad_ = 0;
     }
-    const int frc = check_fault(ws, "mhd_run");
+    const int frc = fault_code(ws, ws->h->fault, "mhd_run");
     if (frc) return frc;
     const int code = status_code(hc.status);
     if (code != MHD_OK) return fail(code, "mhd_run: step loop stopped with status %d after %d steps", hc.status, hc.steps);
@@ -889,9 +903,9 @@ int mhd_diagnostics(mhd_workspace* ws, const mhd_grid* g, double* out6) {
     if (rc) return rc;
     if (!out6) return fail(MHD_ERR_ARG, "mhd_diagnostics: null output");
     g_launches += 2;
-    CK(mhd::launch_diagnostics(dev(g), (int)elem_bytes(g->dtype), ws->gamma, gdx(g), gdy(g), ws->d_diag,
-                               ws->d_diag + 6 * 1024, ws->stream));
-    CK(cudaMemcpyAsync(out6, ws->d_diag + 6 * 1024, 6 * sizeof(double), cudaMemcpyDeviceToHost, ws->stream));
+    CK(mhd::launch_diagnostics(dev(g), (int)elem_bytes(g->dtype), ws->gamma, gdx(g), gdy(g), ws->d->diag,
+                               ws->d->diag + 6 * 1024, ws->stream));
+    CK(cudaMemcpyAsync(out6, ws->d->diag + 6 * 1024, 6 * sizeof(double), cudaMemcpyDeviceToHost, ws->stream));
     CK(cudaStreamSynchronize(ws->stream));
     return MHD_OK;
 }

@@ -206,12 +206,10 @@ cudaError_t launch_argmax_policy(const DevGrid& g, double gamma, double ch, doub
 }
 
 template <class PH>
-cudaError_t launch_max_policy(const DevGrid& g, double gamma, double ch, unsigned long long* out, cudaStream_t st,
-                              int nsm) {
+cudaError_t launch_max_policy(const DevGrid& g, double gamma, double ch, const MaxOut& out, cudaStream_t st) {
     const long long n = (long long)g.nx * g.ny;
     long long blocks = (n + 255) / 256;
-    const long long cap = (long long)nsm * 8;
-    if (blocks > cap) blocks = cap;
+    if (blocks > 8LL * kSMs) blocks = 8LL * kSMs;
     if (blocks < 1) blocks = 1;
     max_speed_kernel<PH><<<(unsigned)blocks, 256, 0, st>>>(g, gamma, ch, out);
     return cudaGetLastError();

@@ -83,11 +83,9 @@ cudaError_t launch_faces_f64(const double* UL, const double* UR, long long n, in
 cudaError_t launch_faces_f32(const double* UL, const double* UR, long long n, int dir, int solver, double ch,
                              double gamma, double* F, cudaStream_t st);
 
-// CFL maximum (floored by ch) folded into *out with atomicMax on the bits.
-cudaError_t launch_max_speed_f64(const DevGrid& g, double gamma, double ch, unsigned long long* out,
-                                 cudaStream_t st, int nsm);
-cudaError_t launch_max_speed_f32(const DevGrid& g, double gamma, double ch, unsigned long long* out,
-                                 cudaStream_t st, int nsm);
+// CFL maximum of a state (floored by ch), delivered as `out` says.
+cudaError_t launch_max_speed_f64(const DevGrid& g, double gamma, double ch, const MaxOut& out, cudaStream_t st);
+cudaError_t launch_max_speed_f32(const DevGrid& g, double gamma, double ch, const MaxOut& out, cudaStream_t st);
 
 // Smallest linear interior index whose CFL speed (floor ch) equals m (atomicMin on *idx).
 cudaError_t launch_argmax_f64(const DevGrid& g, double gamma, double ch, double m, int* idx, cudaStream_t st);
@@ -117,8 +115,5 @@ cudaError_t launch_initialise(const DevGrid& g, int elem_bytes, int id, double x
 // Parametrised Orszag-Tang initial data (mhd_initialise_orszag_tang).
 cudaError_t launch_initialise_ot(const DevGrid& g, int elem_bytes, double b0, double gamma, const double* amp,
                                  double x0, double y0, double dx, double dy, cudaStream_t st);
-
-// Clock initialisation: maxbits[0] = bits(max0), maxbits[1] = 0, t = 0, steps = 0.
-cudaError_t launch_clock_init(DevClock* c, const unsigned long long* max0, cudaStream_t st);
 
 }  // namespace mhd

@@ -83,6 +83,18 @@ struct DevClock {
     double* log;         // {dt, ch, damp} of each step taken, when non-null
 };
 
+// Where a standalone CFL maximum goes: bits in slot 0 of a fresh clock (with its
+// log), or bits and the fault word to page-locked host memory.  acc and count
+// (device, zero between launches) are the reduction's own.
+struct MaxOut {
+    unsigned long long* acc;
+    unsigned* count;
+    DevClock* clock;
+    double* log;
+    unsigned long long* host;
+    const int* fault;
+};
+
 enum ClockStatus : int {
     CLK_OK = 0,
     CLK_NO_SPEED = 1,     // max wave speed <= 0 (the reference throws, solver_cpu.cpp:304-306)

@@ -117,9 +117,8 @@ cudaError_t launch_argmax_f64(const DevGrid& g, double gamma, double ch, double 
     return launch_argmax_policy<ExactPolicy<HLL, MINMOD>>(g, gamma, ch, m, idx, st);
 }
 
-cudaError_t launch_max_speed_f64(const DevGrid& g, double gamma, double ch, unsigned long long* out,
-                                 cudaStream_t st, int nsm) {
-    return launch_max_policy<ExactPolicy<HLL, MINMOD>>(g, gamma, ch, out, st, nsm);
+cudaError_t launch_max_speed_f64(const DevGrid& g, double gamma, double ch, const MaxOut& out, cudaStream_t st) {
+    return launch_max_policy<ExactPolicy<HLL, MINMOD>>(g, gamma, ch, out, st);
 }
 
 }  // namespace mhd

@@ -762,11 +762,13 @@ __global__ void __launch_bounds__(32 * PH::kYWarps, PH::kYBlocks) sweep_y_kernel
 }
 
 // Standalone CFL maximum over the interior (compute_dt, src/cpu/solver_cpu.cpp:283-303)
-// with `ch` as the floor; one atomic per warp.
+// with `ch` as the floor; one atomic per CTA.  The last CTA delivers the result
+// (MaxOut) and leaves acc and count at zero for the next launch, so a caller needs
+// no memset, no clock set-up launch and no copy.
 template <class PH>
-__global__ void __launch_bounds__(256) max_speed_kernel(DevGrid gd, double gamma, double ch,
-                                                       unsigned long long* out) {
+__global__ void __launch_bounds__(256) max_speed_kernel(DevGrid gd, double gamma, double ch, MaxOut out) {
     using R = typename PH::Real;
+    __shared__ double part[8];
     const long long n = (long long)gd.nx * gd.ny;
     double vmax = 0.0;
     for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n;
@@ -782,7 +784,25 @@ __global__ void __launch_bounds__(256) max_speed_kernel(DevGrid gd, double gamma
         const double t = __shfl_xor_sync(FULL, vmax, o);
         vmax = (vmax < t) ? t : vmax;
     }
-    if ((threadIdx.x & 31) == 0) atomic_max_pos(out, vmax);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = vmax;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < 8; ++w) vmax = (vmax < part[w]) ? part[w] : vmax;
+    atomic_max_pos(out.acc, vmax);
+    __threadfence();
+    if (atomicInc(out.count, gridDim.x - 1) != gridDim.x - 1) return;
+    const unsigned long long mx = atomicExch(out.acc, 0ull);
+    if (out.clock) {
+        DevClock c{};  // t = 0, no steps, running
+        c.maxbits[0] = mx;
+        c.log = out.log;
+        *out.clock = c;
+    }
+    if (out.host) {
+        out.host[0] = mx;
+        out.host[1] = (unsigned long long)*out.fault;
+        __threadfence_system();
+    }
 }
 
 }  // namespace mhd
