@@ -457,14 +457,15 @@ __host__ __device__ inline SweepPlan y_plan(int rows, int per) {
 // len ~ sqrt(N), with the factor `c` measured per sweep and precision and `cap`
 // the longest worth taking (the large-grid lengths, kXRpw and kYBand).  Up to
 // `one_wave` iterations per slot the tasks all run at once, and the shortest
-// length that still fits them in one wave is best (x: 4, y: 8; e.g. FP32 y at
+// length that still fits them in one wave is best (x: 4, y: 11; e.g. FP32 y at
 // 512^2, N = 3.7: 53 / 38 / 37 / 31 / 33 / 36 us with 1 / 2 / 3 / 4 / 5 / 6
-// rows).  Measured (HLLD, van Leer, us; with the cap's length at every size ->
+// rows; at 768^2, N = 8.1, 41.9 us with 9 rows against 49.0 with 5).  Measured
+// (HLLD, van Leer, us; with the cap's length at every size ->
 // by this rule): FP32 x 512^2 35 -> 22, 1024^2 55 -> 48, y 512^2 107 -> 31,
 // 1024^2 121 -> 72, 2048^2 202 -> 183; FP64 x 512^2 64 -> 55, 1024^2 173 -> 160,
 // y 512^2 445 -> 91, 1024^2 454 -> 235, 2048^2 781 -> 687; 64^2 y 106 -> 14 FP32,
 // 423 -> 23 FP64.
-constexpr double kXOneWave = 4.0, kYOneWave = 8.0;
+constexpr double kXOneWave = 4.0, kYOneWave = 11.0;
 struct TaskLen {
     int len;
     bool one_wave;  // equal tasks, no guided tail
