@@ -419,6 +419,12 @@ MHD_HD_INLINE bool physical(const double* V, double u, double v, double w, doubl
            finite_d(w) && finite_d(V[BX]) && finite_d(V[BY]) && finite_d(V[BZ]) && finite_d(V[PSI]);
 }
 
+// The same for a state whose pressure p follows from its conserved values: p is
+// finite only if rho, u, v, w, B (and E) are, so four tests stand for nine.
+MHD_HD_INLINE bool physical_p(const double* V, double p, double floor_p) {
+    return (V[RHO] > kRhoFloor) & finite_d(p) & (p > floor_p) & finite_d(V[PSI]);
+}
+
 // The limited slopes of all fields.
 template <int LIMITER>
 MHD_HD_INLINE void slopes(const double* Wm, const double* Wc, const double* Wp, double* s) {
@@ -456,14 +462,6 @@ MHD_HD_INLINE void reconstruct_of(const double* Wm, const double* Wc, const doub
             Wr[k] = Wc[k] + 0.5 * s[k];
         }
     }
-    if (!physical(Wl, Wl[PU], Wl[PV], Wl[PW], Wl[PP])) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) Wl[k] = Wc[k];
-    }
-    if (!physical(Wr, Wr[PU], Wr[PV], Wr[PW], Wr[PP])) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) Wr[k] = Wc[k];
-    }
     // p / (g - 1) and 1 / rho of both
     const double gm1 = g - 1.0;
     const Recip rg = recip(gm1);
@@ -486,6 +484,23 @@ MHD_HD_INLINE void reconstruct_of(const double* Wm, const double* Wc, const doub
     cons(Wr, er, Ur);
     prim_of(Ul, irl, g, ul, vl, wl, pl);
     prim_of(Ur, irr, g, ur, vr, wr, pr);
+    // A face state with a finite recomputed pressure has every value but psi
+    // finite (an infinity or NaN in any would reach it): physical at once.  The
+    // others take the full test, which fails the face state over to the centre's.
+    if (!((Wl[PP] > kPFloor) & physical_p(Wl, pl, -HUGE_VAL) & (Wr[PP] > kPFloor) & physical_p(Wr, pr, -HUGE_VAL))) {
+        const bool okl = physical(Wl, Wl[PU], Wl[PV], Wl[PW], Wl[PP]), okr = physical(Wr, Wr[PU], Wr[PV], Wr[PW], Wr[PP]);
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            if (!okl) Wl[k] = Wc[k];
+            if (!okr) Wr[k] = Wc[k];
+        }
+        irl = 1.0 / Wl[RHO];
+        irr = 1.0 / Wr[RHO];
+        cons(Wl, Wl[PP] / gm1, Ul);
+        cons(Wr, Wr[PP] / gm1, Ur);
+        prim_of(Ul, irl, g, ul, vl, wl, pl);
+        prim_of(Ur, irr, g, ur, vr, wr, pr);
+    }
     flux_of<DIR>(Ul, ul, vl, wl, pl, ch, Fl);
     flux_of<DIR>(Ur, ur, vr, wr, pr, ch, Fr);
     const double s = 0.5 * dtd;
@@ -502,12 +517,12 @@ MHD_HD_INLINE void reconstruct_of(const double* Wm, const double* Wc, const doub
     R.v[13] = ir2[1];
     prim_of(L.v, L.v[13], g, L.v[9], L.v[10], L.v[11], L.v[12]);
     prim_of(R.v, R.v[13], g, R.v[9], R.v[10], R.v[11], R.v[12]);
-    if (!physical(L.v, L.v[9], L.v[10], L.v[11], L.v[12])) {
+    if (!physical_p(L.v, L.v[12], kPFloor)) {
 #pragma unroll
         for (int k = 0; k < NV; ++k) L.v[k] = Ul[k];
         L.v[9] = ul; L.v[10] = vl; L.v[11] = wl; L.v[12] = pl; L.v[13] = irl;
     }
-    if (!physical(R.v, R.v[9], R.v[10], R.v[11], R.v[12])) {
+    if (!physical_p(R.v, R.v[12], kPFloor)) {
 #pragma unroll
         for (int k = 0; k < NV; ++k) R.v[k] = Ur[k];
         R.v[9] = ur; R.v[10] = vr; R.v[11] = wr; R.v[12] = pr; R.v[13] = irr;
