@@ -137,16 +137,12 @@ __device__ __forceinline__ void atomic_max_pos(unsigned long long* addr, double 
     if (v > 0.0) atomicMax(addr, (unsigned long long)__double_as_longlong(v));
 }
 
-// dt / ch / damping for this step, computed identically by every thread.
-// Returns false when the step must be skipped.  Mirrors the driver loop of
-// scripts/cpu/main_cpu.cpp:196-216 and compute_dt (src/cpu/solver_cpu.cpp:304-311).
-__device__ __forceinline__ bool step_scalars(const StepParams& P, double& dt, double& ch, double& damp) {
-    if (P.clock == nullptr) {
-        dt = P.dt; ch = P.ch; damp = P.damp;
-        return true;
-    }
+// dt / ch / damping of a device-mode step from the clock's slots, which no launch of
+// the step changes: a thread that forms them again after its march gets the same
+// values, whatever has become of the clock's status meanwhile (a bounded wait that
+// gives up sets it while the sweep runs).  False when there is no such step.
+__device__ __forceinline__ bool clock_scalars(const StepParams& P, double& dt, double& ch, double& damp) {
     const DevClock* c = P.clock;
-    if (*(volatile const int*)&c->status != CLK_OK) return false;
     const double t = *(volatile const double*)&c->t[P.parity];
     if (!(t < P.t_end)) return false;
     const double mx = __longlong_as_double(
@@ -160,6 +156,18 @@ __device__ __forceinline__ bool step_scalars(const StepParams& P, double& dt, do
     if (dt < P.dt_min) return false;
     damp = exp(-dt * ch / P.cr);
     return true;
+}
+
+// dt / ch / damping for this step, computed identically by every thread.
+// Returns false when the step must be skipped.  Mirrors the driver loop of
+// scripts/cpu/main_cpu.cpp:196-216 and compute_dt (src/cpu/solver_cpu.cpp:304-311).
+__device__ __forceinline__ bool step_scalars(const StepParams& P, double& dt, double& ch, double& damp) {
+    if (P.clock == nullptr) {
+        dt = P.dt; ch = P.ch; damp = P.damp;
+        return true;
+    }
+    if (*(volatile const int*)&P.clock->status != CLK_OK) return false;
+    return clock_scalars(P, dt, ch, damp);
 }
 
 // The step's c_h again, for a use after a march (the y-sweep runs at its register

@@ -713,11 +713,13 @@ __device__ __forceinline__ void y_fold(const StepParams& P, double vmax, unsigne
 
 // Clock advance of a completed device-mode step (one thread per step).
 // The scalars are formed again rather than held across the march, which runs at
-// its register limit; the slots they come from do not change during the step.
+// its register limit; the slots they come from do not change during the step,
+// but the status may (a wait of the TMA-staged sweep that gave up), so it is not
+// looked at here: such a step advances the clock by its own dt and c_h.
 __device__ __forceinline__ void clock_advance(const StepParams& P) {
     DevClock* c = P.clock;
     double dt, ch, damp;
-    step_scalars(P, dt, ch, damp);
+    if (!clock_scalars(P, dt, ch, damp)) return;  // not for a step that began
     if (c->log) {
         double* l = c->log + 3 * c->steps;
         l[0] = dt; l[1] = ch; l[2] = damp;
