@@ -408,7 +408,14 @@ int mhd_workspace_create(const mhd_grid* g, mhd_workspace** out) {
         mhd_workspace_destroy(ws);
         return fail(MHD_ERR_NOMEM, "mhd_workspace_create: device scratch");
     }
-    cudaMemset(ws->d, 0, offsetof(mhd_workspace::Device, diag));
+    // zero before any launch on whatever stream the workspace is given (a
+    // non-blocking one does not wait for the default stream)
+    cudaError_t e = cudaMemsetAsync(ws->d, 0, offsetof(mhd_workspace::Device, diag), nullptr);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+    if (e != cudaSuccess) {
+        mhd_workspace_destroy(ws);
+        return fail(MHD_ERR_CUDA, "mhd_workspace_create: %s", cudaGetErrorString(e));
+    }
     *out = ws;
     return MHD_OK;
 }
