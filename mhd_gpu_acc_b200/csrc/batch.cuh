@@ -135,6 +135,17 @@ __global__ void __launch_bounds__(32 * YS_WARPS, PH::kYBlocks)
 // maxbits[0] of its clock, which starts at 0: CTAs of 256 threads take
 // kMaxUnit cells of one instance each, one atomic per CTA.
 constexpr int kMaxUnit = 4096;
+// Unit k of an instance: n cells in row order from column i0 of row j0 on (an
+// instance may have 2^31 cells and more).
+__host__ __device__ __forceinline__ long long max_units(const DevGrid& g) {
+    return ((long long)g.nx * g.ny + kMaxUnit - 1) / kMaxUnit;
+}
+__host__ __device__ __forceinline__ void max_unit(const DevGrid& g, int k, int& i0, int& j0, int& n) {
+    const long long c0 = (long long)k * kMaxUnit, left = (long long)g.nx * g.ny - c0;
+    j0 = c0 <= 0xffffffffLL ? (int)((unsigned)c0 / (unsigned)g.nx) : (int)(c0 / g.nx);
+    i0 = (int)(c0 - (long long)j0 * g.nx);
+    n = left < kMaxUnit ? (int)left : kMaxUnit;
+}
 template <class PH>
 __global__ void __launch_bounds__(256) batch_max_kernel(const BatchInst* __restrict__ inst,
                                                        const BatchSeg* __restrict__ seg,
@@ -146,12 +157,13 @@ __global__ void __launch_bounds__(256) batch_max_kernel(const BatchInst* __restr
     const BatchInst& I = inst[s.inst];
     const DevGrid g = I.U;
     const double gamma = I.P.gamma, floor_ch = ch[s.inst];
-    const int c0 = ((int)blockIdx.x - s.unit) * kMaxUnit, c1 = min(s.hi, c0 + kMaxUnit);
+    int i0, j0, n;
+    max_unit(g, (int)blockIdx.x - s.unit, i0, j0, n);
     double vmax = 0.0;
-    for (int c = c0 + threadIdx.x; c < c1; c += 256) {
-        const int j = c / g.nx, i = c - j * g.nx;
+    for (int c = threadIdx.x; c < n; c += 256) {
+        const unsigned q = (unsigned)i0 + c, dj = q / (unsigned)g.nx;
         R U[NV];
-        load_cell(g, g.ng + i, g.ng + j, U);
+        load_cell(g, g.ng + (int)(q - dj * (unsigned)g.nx), g.ng + j0 + (int)dj, U);
         const double v = PH::speed(U, gamma, floor_ch);
         vmax = (vmax < v) ? v : vmax;
     }

@@ -97,7 +97,7 @@ int build_worklist(mhd_batch* b) {
         for (int i = 0; i < n; ++i) {
             const int nx = b->desc[i].nx, ny = b->desc[i].ny, strips = mhd::y_strips(b->host_inst[i].U);
             if (l == 2) {
-                segs.push_back({i, 0, nx * ny, 0, 0, 0, 0, 0, 0});
+                segs.push_back({i, 0, 0, 0, 0, 0, 0, 0, 0});
                 continue;
             }
             const bool by_size = l == 0 ? b->by_size_x : b->by_size_y;
@@ -128,7 +128,7 @@ int build_worklist(mhd_batch* b) {
         std::vector<char> led(n, 0);
         for (auto s = begin; s != segs.end(); ++s) {
             const long long count = l < 2 ? ((long long)s->n * s->width + mhd::YS_WARPS - 1) / mhd::YS_WARPS
-                                          : ((long long)s->hi + mhd::kMaxUnit - 1) / mhd::kMaxUnit;
+                                          : mhd::max_units(b->host_inst[s->inst].U);
             s->lead = !led[s->inst];
             led[s->inst] = 1;
             s->unit = (int)(units.size() - unit0[l]);

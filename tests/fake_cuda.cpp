@@ -20,7 +20,7 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
     return cudaSuccess;
 }
 cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t st) {
-    fake::put(st, [=] { if (!fake::hollow || n <= (1u << 20)) std::memset(p, v, n); });
+    fake::put(st, [=] { if (!fake::hollow || n <= (1u << 30)) std::memset(p, v, n); });
     return cudaSuccess;
 }
 cudaError_t cudaMemset(void* p, int v, size_t n) { return cudaMemsetAsync(p, v, n, nullptr); }

@@ -21,7 +21,7 @@ inline std::vector<std::function<void()>> queued;  // on the default stream
 inline std::map<char*, size_t> device, host;       // live allocations
 inline int mallocs = 0, host_allocs = 0, fail_malloc_at = -1;
 inline bool fail_host = false;
-inline bool hollow = false;  // device blocks over 1 MB get a page only (their contents are not looked at)
+inline bool hollow = false;  // device blocks over 1 GB get a page only (their contents are not looked at)
 
 inline void drain() {
     std::lock_guard<std::recursive_mutex> g(lock);
@@ -43,7 +43,7 @@ inline bool in(const std::map<char*, size_t>& m, const void* p, size_t n) {
 }
 inline cudaError_t alloc(std::map<char*, size_t>& m, void** p, size_t n) {
     std::lock_guard<std::recursive_mutex> g(lock);
-    const size_t real = hollow && n > (1u << 20) ? 4096 : n;
+    const size_t real = hollow && n > (1u << 30) ? 4096 : n;
     *p = std::malloc(real ? real : 1);
     std::memset(*p, 0xab, real);
     m[(char*)*p] = n;
