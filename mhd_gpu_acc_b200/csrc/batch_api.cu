@@ -17,6 +17,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <exception>
 #include <string>
 #include <vector>
 
@@ -77,8 +78,10 @@ cudaError_t phase(mhd_batch* b, int parity, int which, cudaStream_t st) {
                                : mhd::launch_batch_f32(b->d_inst, list, b->d_ch, b->n, parity, which, b->solver, b->limiter, ctas, st);
 }
 
-// Work lists for the current shape; uploads the tables and drops the graph.
-int build_worklist(mhd_batch* b) {
+// Work lists for the current shape; uploads the tables and drops the graph.  Without
+// memory for a longer table the lists, and the graph that holds their addresses,
+// stay as they were.
+int build_worklist(mhd_batch* b) try {
     const int n = b->n;
     long long x_work = 0, y_work = 0;
     for (int i = 0; i < n; ++i) {
@@ -142,16 +145,21 @@ int build_worklist(mhd_batch* b) {
         b->host_inst[n + i] = b->host_inst[i];
         b->host_inst[n + i].P.parity = 1;
     }
-    if (units.size() > b->units_cap) {
-        if (b->d_units) cudaFree(b->d_units);
-        b->d_units = nullptr;
-        b->units_cap = 0;
-        if (cudaMalloc(&b->d_units, sizeof(int) * units.size()) != cudaSuccess) {
-            b->d_units = nullptr;
-            return berr(MHD_ERR_NOMEM, "batch: work list");
-        }
+    int* d_units = b->d_units;
+    if (units.size() > b->units_cap && cudaMalloc(&d_units, sizeof(int) * units.size()) != cudaSuccess) {
+        cudaGetLastError();
+        return berr(MHD_ERR_NOMEM, "batch: work list");
+    }
+    if (b->graph) {
+        cudaGraphExecDestroy(b->graph);
+        b->graph = nullptr;
+    }
+    if (d_units != b->d_units) {
+        if (b->d_units) cudaFree(b->d_units);  // waits for launches that read it
+        b->d_units = d_units;
         b->units_cap = units.size();
     }
+    for (auto& l : b->lists) l = {};  // no units until the tables are there
     BCK(cudaMemcpyAsync(b->d_inst, b->host_inst.data(), sizeof(mhd::BatchInst) * b->host_inst.size(),
                         cudaMemcpyHostToDevice, b->stream));
     BCK(cudaMemcpyAsync(b->d_seg, segs.data(), sizeof(mhd::BatchSeg) * segs.size(), cudaMemcpyHostToDevice, b->stream));
@@ -159,11 +167,9 @@ int build_worklist(mhd_batch* b) {
     BCK(cudaStreamSynchronize(b->stream));
     for (int l = 0; l < 3; ++l)
         b->lists[l] = {b->d_seg + seg0[l], b->d_units + unit0[l], (int)(unit0[l + 1] - unit0[l])};
-    if (b->graph) {
-        cudaGraphExecDestroy(b->graph);
-        b->graph = nullptr;
-    }
     return MHD_OK;
+} catch (const std::exception& e) {
+    return berr(MHD_ERR_NOMEM, e.what());
 }
 
 // Every clock from its instance's CFL maximum (floored by the carried c_h).
@@ -308,10 +314,18 @@ int mhd_batch_set_tuning(mhd_batch* b, const mhd_batch_tuning* t) {
     if (!b || !t) return berr(MHD_ERR_ARG, "mhd_batch_set_tuning: null argument");
     if (t->xrpw < 1 || t->xrpw > 64 || t->yseg < 4 || t->yseg > 4096 || t->ctas_x < 0 || t->ctas_y < 0)
         return berr(MHD_ERR_ARG, "mhd_batch_set_tuning: out of range");
+    const mhd_batch_tuning tune = b->tune;
+    const bool by_size_x = b->by_size_x, by_size_y = b->by_size_y;
     b->tune = *t;
     b->by_size_x = b->by_size_y = false;
     default_ctas(b);
-    return build_worklist(b);
+    const int rc = build_worklist(b);
+    if (rc) {  // the lists are still the former ones
+        b->tune = tune;
+        b->by_size_x = by_size_x;
+        b->by_size_y = by_size_y;
+    }
+    return rc;
 }
 
 int mhd_batch_run(mhd_batch* b, int max_steps, mhd_run_info* info) {
@@ -392,15 +406,10 @@ int mhd_batch_tune_candidates(int which, int* out, int cap) {
     return n;
 }
 
-int mhd_batch_tune(mhd_batch* b, int reps, mhd_batch_tuning* best_out) {
-    mhd::NvtxRange nvtx_range("mhd_batch_tune");
-    if (!b) return berr(MHD_ERR_STATE, "mhd_batch_tune: null batch");
-    if (reps < 1) reps = 3;
+// The tuner's search between its events: leaves the lists of the best shape.
+static int tune_shapes(mhd_batch* b, int reps, cudaEvent_t e0, cudaEvent_t e1) {
     int rc = start_clocks(b);
     if (rc) return rc;
-    cudaEvent_t e0, e1;
-    BCK(cudaEventCreate(&e0));
-    BCK(cudaEventCreate(&e1));
     mhd_batch_tuning best = b->tune;
     const auto& xr = kTuneXrpw;
     const auto& xc = kTuneCtasPerSm;
@@ -453,11 +462,30 @@ int mhd_batch_tune(mhd_batch* b, int reps, mhd_batch_tuning* best_out) {
     if ((rc = build_worklist(b))) return rc;
     if ((rc = time_phase(2, &ms))) return rc;
     b->by_size_y = ms < best_ms;
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
     b->tune = best;
-    if ((rc = build_worklist(b))) return rc;
-    if (best_out) *best_out = best;
+    return build_worklist(b);
+}
+
+int mhd_batch_tune(mhd_batch* b, int reps, mhd_batch_tuning* best_out) {
+    mhd::NvtxRange nvtx_range("mhd_batch_tune");
+    if (!b) return berr(MHD_ERR_STATE, "mhd_batch_tune: null batch");
+    const mhd_batch_tuning tune = b->tune;
+    const bool by_size_x = b->by_size_x, by_size_y = b->by_size_y;
+    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    int rc = cudaEventCreate(&e0) == cudaSuccess && cudaEventCreate(&e1) == cudaSuccess
+                 ? tune_shapes(b, reps < 1 ? 3 : reps, e0, e1)
+                 : berr(MHD_ERR_CUDA, "mhd_batch_tune: events");
+    if (e0) cudaEventDestroy(e0);
+    if (e1) cudaEventDestroy(e1);
+    if (rc) {  // back to the shape that was there (its lists fit the tables)
+        b->tune = tune;
+        b->by_size_x = by_size_x;
+        b->by_size_y = by_size_y;
+        const std::string what = mhd_last_error();
+        build_worklist(b);
+        return berr(rc, what.c_str());
+    }
+    if (best_out) *best_out = b->tune;
     return MHD_OK;
 }
 

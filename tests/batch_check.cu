@@ -3,6 +3,7 @@
 // test_batch_lists.py, no GPU).  The fake launches look through the lists they are
 // given, which have to lie in live device memory, as the kernels would.
 //   large: instances about and past 2^31 cells.
+//   no_memory: a longer work list that finds no memory leaves the batch as it was.
 #include <cstdio>
 
 #include "../include/mhd_b200.h"
@@ -18,6 +19,7 @@ struct Launch {
     std::vector<mhd::BatchSeg> seg;  // of each unit
 };
 static std::vector<Launch> launches;
+static std::function<void(const mhd::BatchInst*, const mhd::BatchList&, int, bool)> on_launch;
 
 static void look(const mhd::BatchInst* inst, const mhd::BatchList& list, int n, int which, int ctas) {
     if (which == 0) return;
@@ -56,13 +58,15 @@ static void look(const mhd::BatchInst* inst, const mhd::BatchList& list, int n, 
 
 namespace mhd {
 cudaError_t launch_batch_f32(const BatchInst* inst, const BatchList& list, const double*, int n, int, int which, int, int,
-                             int ctas, cudaStream_t) {
+                             int ctas, cudaStream_t st) {
     look(inst, list, n, which, ctas);
+    if (on_launch && which > 0) on_launch(inst, list, which, st == (cudaStream_t)8);
     return cudaSuccess;
 }
 cudaError_t launch_batch_f64(const BatchInst* inst, const BatchList& list, const double*, int n, int, int which, int, int,
-                             int ctas, cudaStream_t) {
+                             int ctas, cudaStream_t st) {
     look(inst, list, n, which, ctas);
+    if (on_launch && which > 0) on_launch(inst, list, which, st == (cudaStream_t)8);
     return cudaSuccess;
 }
 void batch_task_lens_f32(long long x, long long y, TaskLen& tx, TaskLen& ty) {
@@ -102,7 +106,48 @@ static void large() {
     fake::hollow = false;
 }
 
+static void no_memory() {
+    std::vector<mhd_instance_desc> d = {desc(1300, 1301), desc(61, 517), desc(4, 4)};
+    mhd_batch* b = nullptr;
+    CHECK(mhd_batch_create(d.data(), 3, MHD_F64, MHD_HLLD, MHD_LIMITER_VANLEER, &b) == MHD_OK);
+    auto run = [&] {  // every launch, the captured graph's among them, on live lists that cover the grids
+        launches.clear();
+        mhd_run_info info[3];
+        CHECK(mhd_batch_run(b, 3, info) == MHD_OK);
+        return launches.back().units;
+    };
+    mhd::BatchInst* inst = nullptr;
+    std::vector<std::pair<int, mhd::BatchList>> captured;
+    on_launch = [&](const mhd::BatchInst* i, const mhd::BatchList& l, int which, bool graph) {
+        inst = const_cast<mhd::BatchInst*>(i);
+        if (graph) captured.push_back({which, l});
+    };
+    fake::graph_launch = [&] {
+        CHECK(captured.size() >= 4);
+        for (size_t k = captured.size() - 4; k < captured.size(); ++k) look(inst, captured[k].second, 3, captured[k].first, 0);
+    };
+    const int units = run();
+    mhd_batch_tuning was{}, now{};
+    CHECK(mhd_batch_get_tuning(b, &was) == MHD_OK);
+    const mhd_batch_tuning fine{1, 4, 0, 0};
+    for (int k = 0; k < 2; ++k) {  // through set_tuning and through the tuner
+        fake::fail_malloc_at = fake::mallocs;
+        CHECK((k == 0 ? mhd_batch_set_tuning(b, &fine) : mhd_batch_tune(b, 1, nullptr)) == MHD_ERR_NOMEM);
+        fake::fail_malloc_at = -1;
+        CHECK(mhd_batch_get_tuning(b, &now) == MHD_OK && std::memcmp(&was, &now, sizeof now) == 0);
+        CHECK(run() == units && launches.back().ctas == 0);
+    }
+    CHECK(mhd_batch_set_tuning(b, &fine) == MHD_OK && run() > units);
+    CHECK(mhd_batch_tune(b, 1, nullptr) == MHD_OK);
+    run();
+    on_launch = nullptr;
+    fake::graph_launch = nullptr;
+    CHECK(mhd_batch_destroy(b) == MHD_OK);
+    CHECK(fake::device.empty());
+}
+
 int main() {
+    no_memory();
     large();
     std::printf("%d failures\n", failures);
     return failures ? 1 : 0;
