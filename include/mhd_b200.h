@@ -323,9 +323,11 @@ typedef struct mhd_instance_desc {
     double gamma, cfl, cr, t_end;
 } mhd_instance_desc;
 /* Launch shape of the batched sweeps: x-sweep work per warp (xrpw: row
- * segments of 128 * xrpw - 4 cells), y-sweep segment length, persistent CTAs
- * of each phase (0 = default from the SM count).  A batch that was never tuned
- * takes the lengths that suit its size and deals the work out dynamically. */
+ * segments of 128 * xrpw - 4 cells), y-sweep segment length, resident CTAs
+ * of each phase (0 = default from the SM count).  A phase at its default values (x:
+ * xrpw 8, ctas_x 0; y: yseg 64, ctas_y 0), as in a batch that was never tuned,
+ * takes the lengths that suit the size of the batch and deals the work out
+ * dynamically. */
 typedef struct mhd_batch_tuning {
     int xrpw, yseg, ctas_x, ctas_y;
 } mhd_batch_tuning;
@@ -347,9 +349,9 @@ int mhd_batch_get_tuning(const mhd_batch* b, mhd_batch_tuning* t);
 int mhd_batch_set_tuning(mhd_batch* b, const mhd_batch_tuning* t);
 /* Autotuner: times each sweep phase for every candidate launch shape (x work
  * per warp xrpw 2/4/8/16 x 2-4 CTAs per SM; y segment 16/24/32/48/64/128 x 2-4
- * CTAs per SM) on the batch's current states, `reps` launches each, and the
- * untuned shape, and keeps the fastest of each phase (*best: the fastest
- * candidate).  Leaves the instances one step ahead. */
+ * CTAs per SM; the default values among them) on the batch's current states,
+ * `reps` launches each, and keeps the fastest of each phase, which *best
+ * reproduces in mhd_batch_set_tuning.  Leaves the instances one step ahead. */
 int mhd_batch_tune(mhd_batch* b, int reps, mhd_batch_tuning* best);
 /* The autotuner's candidate values: which = 0 x work per warp (xrpw), 1 y
  * segment lengths, 2 CTAs per SM (both phases).  Copies up to cap of them into

@@ -18,8 +18,11 @@
 // instances of 64..1024 cells a side (29.5M cells, FP32 HLLD, van Leer) x 1.21 ->
 // 0.89 ms and y 1.99 -> 1.19 ms against 444 CTAs striding over the list in fixed
 // order with one task length (kDefaultBatchXRpw, kDefaultYSeg; of the y gain 0.2 ms
-// is the ghost scatter's).  An explicit tuning keeps that form.
+// is the ghost scatter's).  An explicit tuning sets the task lengths, how many of
+// the x CTAs are resident at a time, and the CTAs that stride over the y list.
 #pragma once
+
+#include <algorithm>
 
 #include "dispatch.cuh"
 
@@ -56,35 +59,33 @@ __device__ __forceinline__ bool seg_task(const BatchSeg& s, int task, int& idx, 
 template <class PH>
 constexpr int bx_smem_bytes() { return BX_WARPS * XRing<PH>::kWarpBytes; }
 
-// STRIDE: the CTAs stride over the list (an explicit tuning); else CTA u takes unit
-// u, which leaves the march the loop's registers (without them it spills 8 bytes:
-// 908 -> 892 us at 96 instances of 64..1024 cells a side).
-template <class PH, bool STRIDE>
+// CTA u takes unit u, under any tuning: with a loop over units the march spills 8
+// bytes (908 against 892 us at 96 instances of 64..1024 cells a side), and a second
+// kernel with the loop contracts other FP32 multiply-adds, which would make results
+// depend on the launch shape.
+template <class PH>
 __global__ void __launch_bounds__(32 * BX_WARPS, PH::kXBlocks)
-    batch_x_kernel(const BatchInst* __restrict__ inst, const BatchSeg* __restrict__ seg, const int* __restrict__ unit_seg,
-                   int total) {
+    batch_x_kernel(const BatchInst* __restrict__ inst, const BatchSeg* __restrict__ seg, const int* __restrict__ unit_seg) {
     using V = typename Slot16<typename PH::Real>::V;
     extern __shared__ __align__(16) unsigned char bx_smem[];
     const int warp = threadIdx.x >> 5;
     V* ring = reinterpret_cast<V*>(bx_smem + warp * XRing<PH>::kWarpBytes);
-    for (int u = blockIdx.x; u < total; u = STRIDE ? u + gridDim.x : total) {
-        const BatchSeg s = seg[__ldg(unit_seg + u)];
-        const int local = u - s.unit;
-        const bool lead = s.lead && local == 0 && threadIdx.x == 0;
-        const StepParams& P = inst[s.inst].P;
-        double dt, ch, damp;
-        if (!step_scalars(P, dt, ch, damp)) {
-            if (lead) clock_flag_skip(P);
-            continue;
-        }
-        if (lead) P.clock->maxbits[P.parity ^ 1] = 0ull;
-        int row, c0, len;
-        if (seg_task(s, local * BX_WARPS + warp, row, c0, len)) {  // whole warp
-            const DevGrid in = inst[s.inst].U;
-            DevGrid out = in;
-            out.data = inst[s.inst].T;
-            x_segment<PH>(in, out, P, dt, ch, in.ng + row, c0, len, ring);
-        }
+    const BatchSeg s = seg[__ldg(unit_seg + blockIdx.x)];
+    const int local = (int)blockIdx.x - s.unit;
+    const bool lead = s.lead && local == 0 && threadIdx.x == 0;
+    const StepParams& P = inst[s.inst].P;
+    double dt, ch, damp;
+    if (!step_scalars(P, dt, ch, damp)) {
+        if (lead) clock_flag_skip(P);
+        return;
+    }
+    if (lead) P.clock->maxbits[P.parity ^ 1] = 0ull;
+    int row, c0, len;
+    if (seg_task(s, local * BX_WARPS + warp, row, c0, len)) {  // whole warp
+        const DevGrid in = inst[s.inst].U;
+        DevGrid out = in;
+        out.data = inst[s.inst].T;
+        x_segment<PH>(in, out, P, dt, ch, in.ng + row, c0, len, ring);
     }
 }
 
@@ -180,6 +181,14 @@ __global__ void __launch_bounds__(256) batch_max_kernel(const BatchInst* __restr
     }
 }
 
+// Dynamic shared memory of an x phase of which `ctas` CTAs (0: as many as fit) are
+// to be resident at a time: an even share of the SM for each.
+template <class PH>
+int bx_smem_of(int ctas) {
+    const int per_sm = ctas > 0 ? std::max(1, ctas / kSMs) : PH::kXBlocks;
+    return per_sm < PH::kXBlocks ? kSmemPerSM / per_sm - kSmemPerCTAReserve : bx_smem_bytes<PH>();
+}
+
 // The x phase's dynamic shared memory opt-in (once per policy and device,
 // before any stream capture: mhd_batch_run makes a which = 0 call first).
 template <class PH>
@@ -188,12 +197,10 @@ cudaError_t bx_setup() {
                   "batched x-phase rings of kXBlocks CTAs exceed an SM's shared memory");
     static PerDeviceOnce once;
     return once.run([] {
-        cudaError_t r = cudaSuccess;
-        for (auto* k : {batch_x_kernel<PH, false>, batch_x_kernel<PH, true>}) {
-            if (r == cudaSuccess) r = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bx_smem_bytes<PH>());
-            if (r == cudaSuccess)
-                r = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
-        }
+        const auto k = batch_x_kernel<PH>;
+        cudaError_t r = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bx_smem_of<PH>(1));
+        if (r == cudaSuccess)
+            r = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
         // the y phase's window and parameters are a little over the 40 KB of which
         // four CTAs fit the 164 KB split that the runtime picks: ask for the next one,
         // 196 of 228 KB (85 %; more leaves too little L1)
@@ -221,11 +228,10 @@ struct BatchLaunch {
         if (attr != cudaSuccess || which == 0) return attr;  // which 0: the set-up alone
         const BatchInst* I = inst + parity * n;
         const dim3 yb(32, YS_WARPS);
-        constexpr int smem = bx_smem_bytes<PH>();
-        const int grid = ctas > 0 ? ctas : list.units;
-        if (which == 2) batch_y_kernel<PH><<<grid, yb, 0, st>>>(I, list.seg, list.unit_seg, list.units);
-        else if (ctas > 0) batch_x_kernel<PH, true><<<grid, 32 * BX_WARPS, smem, st>>>(I, list.seg, list.unit_seg, list.units);
-        else batch_x_kernel<PH, false><<<grid, 32 * BX_WARPS, smem, st>>>(I, list.seg, list.unit_seg, list.units);
+        if (which == 2)
+            batch_y_kernel<PH><<<ctas > 0 ? ctas : list.units, yb, 0, st>>>(I, list.seg, list.unit_seg, list.units);
+        else
+            batch_x_kernel<PH><<<list.units, 32 * BX_WARPS, bx_smem_of<PH>(ctas), st>>>(I, list.seg, list.unit_seg);
         return cudaGetLastError();
     }
 };

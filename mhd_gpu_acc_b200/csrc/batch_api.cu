@@ -10,9 +10,9 @@
 // phase maps T -> U without touching the clock slots they read, so each phase
 // can be launched repeatedly on unchanged input.  The tuner times every x
 // candidate (rows per warp x persistent CTAs) and then every y candidate
-// (segment length x persistent CTAs) with CUDA events, and the default shape by
-// the size of the batch, keeping the fastest of each phase.  The instances end one
-// step ahead of where they started.
+// (segment length x persistent CTAs) with CUDA events, keeping the fastest of
+// each.  The default values are among the candidates and stand for the shape by the
+// size of the batch.  The instances end one step ahead of where they started.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -56,7 +56,6 @@ struct mhd_batch {
     mhd::BatchList lists[3] = {};
     double* d_ch = nullptr;
     mhd::DevClock* d_clock = nullptr;
-    bool by_size_x = true, by_size_y = true;  // task lengths and CTAs by the size of the batch, not by `tune`
     cudaStream_t stream = nullptr;
     mhd_batch_tuning tune{mhd::kDefaultBatchXRpw, mhd::kDefaultYSeg, 0, 0};
     cudaGraphExec_t graph = nullptr;
@@ -71,8 +70,16 @@ const int kTuneXrpw[] = {2, 4, 8, 16};             // x-sweep rows per warp
 const int kTuneYseg[] = {16, 24, 32, 48, 64, 128};  // y-sweep segment rows
 const int kTuneCtasPerSm[] = {2, 3, 4};             // persistent CTAs per SM, both phases
 
+// A phase at its default tuning takes its lengths by the size of the batch and one
+// CTA per unit; any other tuning is taken as it is.  So the four values say all
+// there is to a shape: those that get_tuning or the tuner give make the same one
+// when they are set, on this batch or another.
+int default_ctas(const mhd_batch* b) { return 3 * b->nsm; }
+bool by_size_x(const mhd_batch* b) { return b->tune.xrpw == mhd::kDefaultBatchXRpw && b->tune.ctas_x == default_ctas(b); }
+bool by_size_y(const mhd_batch* b) { return b->tune.yseg == mhd::kDefaultYSeg && b->tune.ctas_y == default_ctas(b); }
+
 cudaError_t phase(mhd_batch* b, int parity, int which, cudaStream_t st) {
-    const int ctas = which == 1 ? (b->by_size_x ? 0 : b->tune.ctas_x) : which == 2 ? (b->by_size_y ? 0 : b->tune.ctas_y) : 0;
+    const int ctas = which == 1 ? (by_size_x(b) ? 0 : b->tune.ctas_x) : which == 2 ? (by_size_y(b) ? 0 : b->tune.ctas_y) : 0;
     const mhd::BatchList& list = b->lists[which > 0 ? which - 1 : 0];
     return b->dtype == MHD_F64 ? mhd::launch_batch_f64(b->d_inst, list, b->d_ch, b->n, parity, which, b->solver, b->limiter, ctas, st)
                                : mhd::launch_batch_f32(b->d_inst, list, b->d_ch, b->n, parity, which, b->solver, b->limiter, ctas, st);
@@ -103,7 +110,7 @@ int build_worklist(mhd_batch* b) try {
                 segs.push_back({i, 0, 0, 0, 0, 0, 0, 0, 0});
                 continue;
             }
-            const bool by_size = l == 0 ? b->by_size_x : b->by_size_y;
+            const bool by_size = l == 0 ? by_size_x(b) : by_size_y(b);
             const mhd::TaskLen& t = l == 0 ? tx : ty;
             const int cut = by_size && !t.one_wave ? ny - ny / 8 : ny;  // rows from here on in shorter tasks
             for (int p = 0; p < 2; ++p) {
@@ -180,9 +187,9 @@ int start_clocks(mhd_batch* b) {
     return MHD_OK;
 }
 
-void default_ctas(mhd_batch* b) {
-    if (b->tune.ctas_x <= 0) b->tune.ctas_x = 3 * b->nsm;
-    if (b->tune.ctas_y <= 0) b->tune.ctas_y = 3 * b->nsm;
+void fill_ctas(mhd_batch* b) {
+    if (b->tune.ctas_x <= 0) b->tune.ctas_x = default_ctas(b);
+    if (b->tune.ctas_y <= 0) b->tune.ctas_y = default_ctas(b);
 }
 
 }  // namespace
@@ -220,7 +227,7 @@ int mhd_batch_create(const mhd_instance_desc* desc, int n, int dtype, int solver
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&b->nsm, cudaDevAttrMultiProcessorCount, dev);
     if (b->nsm <= 0) b->nsm = 148;
-    default_ctas(b);
+    fill_ctas(b);
     int rc = MHD_OK;
     for (int i = 0; i < n && rc == MHD_OK; ++i) {
         const mhd_instance_desc& d = desc[i];
@@ -315,16 +322,10 @@ int mhd_batch_set_tuning(mhd_batch* b, const mhd_batch_tuning* t) {
     if (t->xrpw < 1 || t->xrpw > 64 || t->yseg < 4 || t->yseg > 4096 || t->ctas_x < 0 || t->ctas_y < 0)
         return berr(MHD_ERR_ARG, "mhd_batch_set_tuning: out of range");
     const mhd_batch_tuning tune = b->tune;
-    const bool by_size_x = b->by_size_x, by_size_y = b->by_size_y;
     b->tune = *t;
-    b->by_size_x = b->by_size_y = false;
-    default_ctas(b);
+    fill_ctas(b);
     const int rc = build_worklist(b);
-    if (rc) {  // the lists are still the former ones
-        b->tune = tune;
-        b->by_size_x = by_size_x;
-        b->by_size_y = by_size_y;
-    }
+    if (rc) b->tune = tune;  // the lists are still the former ones
     return rc;
 }
 
@@ -425,7 +426,6 @@ static int tune_shapes(mhd_batch* b, int reps, cudaEvent_t e0, cudaEvent_t e1) {
         return MHD_OK;
     };
     float best_ms = 1e30f, ms = 0.f;
-    b->by_size_x = false;
     for (int r : xr)
         for (int c : xc) {
             b->tune.xrpw = r;
@@ -440,12 +440,7 @@ static int tune_shapes(mhd_batch* b, int reps, cudaEvent_t e0, cudaEvent_t e1) {
         }
     b->tune.xrpw = best.xrpw;
     b->tune.ctas_x = best.ctas_x;
-    b->by_size_x = true;
-    if ((rc = build_worklist(b))) return rc;
-    if ((rc = time_phase(1, &ms))) return rc;  // T from U
-    b->by_size_x = ms < best_ms;
     best_ms = 1e30f;
-    b->by_size_y = false;
     for (int s : ys)
         for (int c : yc) {
             b->tune.yseg = s;
@@ -458,10 +453,6 @@ static int tune_shapes(mhd_batch* b, int reps, cudaEvent_t e0, cudaEvent_t e1) {
                 best.ctas_y = c * b->nsm;
             }
         }
-    b->by_size_y = true;
-    if ((rc = build_worklist(b))) return rc;
-    if ((rc = time_phase(2, &ms))) return rc;
-    b->by_size_y = ms < best_ms;
     b->tune = best;
     return build_worklist(b);
 }
@@ -470,7 +461,6 @@ int mhd_batch_tune(mhd_batch* b, int reps, mhd_batch_tuning* best_out) {
     mhd::NvtxRange nvtx_range("mhd_batch_tune");
     if (!b) return berr(MHD_ERR_STATE, "mhd_batch_tune: null batch");
     const mhd_batch_tuning tune = b->tune;
-    const bool by_size_x = b->by_size_x, by_size_y = b->by_size_y;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     int rc = cudaEventCreate(&e0) == cudaSuccess && cudaEventCreate(&e1) == cudaSuccess
                  ? tune_shapes(b, reps < 1 ? 3 : reps, e0, e1)
@@ -479,8 +469,6 @@ int mhd_batch_tune(mhd_batch* b, int reps, mhd_batch_tuning* best_out) {
     if (e1) cudaEventDestroy(e1);
     if (rc) {  // back to the shape that was there (its lists fit the tables)
         b->tune = tune;
-        b->by_size_x = by_size_x;
-        b->by_size_y = by_size_y;
         const std::string what = mhd_last_error();
         build_worklist(b);
         return berr(rc, what.c_str());

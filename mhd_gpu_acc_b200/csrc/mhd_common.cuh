@@ -52,8 +52,8 @@ MHD_HD_RULE bool star_degenerate(float d, float rho, float un, float S, float SM
     return fabsf(d) <= kStarDegenRel * (rho * m * m + Bn * Bn);
 }
 constexpr int kDefaultXRpw = 0;  // x-sweep work per warp: 0 = by the size of the launch
-constexpr int kDefaultBatchXRpw = 8;  // batched x-sweep work per warp before tuning
-constexpr int kDefaultYSeg = 64; // batched y-sweep rows per warp segment
+constexpr int kDefaultBatchXRpw = 8;  // batched x-sweep work per warp: with the default CTAs, by the size of the batch
+constexpr int kDefaultYSeg = 64; // batched y-sweep rows per warp segment: the same
 constexpr int kDefaultYBand = 0;  // single-grid y-sweep rows per warp band: 0 = by the size of the launch
 
 struct DevGrid {

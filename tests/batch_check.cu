@@ -3,6 +3,8 @@
 // test_batch_lists.py, no GPU).  The fake launches look through the lists they are
 // given, which have to lie in live device memory, as the kernels would.
 //   large: instances about and past 2^31 cells.
+//   round_trip: the values that get_tuning and the tuner give make the shape that
+//   is in force when they are set, on the same batch and on another.
 //   no_memory: a longer work list that finds no memory leaves the batch as it was.
 #include <cstdio>
 
@@ -79,6 +81,15 @@ void batch_task_lens_f64(long long x, long long y, TaskLen& tx, TaskLen& ty) {
 }
 }  // namespace mhd
 
+static std::vector<int> shape_of_launches() {  // units, CTAs and the lengths of every segment
+    std::vector<int> v;
+    for (const Launch& l : launches) {
+        v.insert(v.end(), {l.which, l.units, l.ctas});
+        for (const mhd::BatchSeg& s : l.seg) v.push_back(s.len);
+    }
+    return v;
+}
+
 static mhd_instance_desc desc(int nx, int ny) {
     mhd_instance_desc d{};
     d.nx = nx;
@@ -146,7 +157,36 @@ static void no_memory() {
     CHECK(fake::device.empty());
 }
 
+static void round_trip() {
+    const std::vector<mhd_instance_desc> d = {desc(1300, 1301), desc(61, 517)};
+    for (int kind = 0; kind < 4; ++kind) {  // untuned, tuned, explicit, explicit in one phase
+        mhd_batch *b = nullptr, *other = nullptr;
+        CHECK(mhd_batch_create(d.data(), 2, MHD_F32, MHD_HLLD, MHD_LIMITER_VANLEER, &b) == MHD_OK);
+        CHECK(mhd_batch_create(d.data(), 2, MHD_F32, MHD_HLLD, MHD_LIMITER_VANLEER, &other) == MHD_OK);
+        const mhd_batch_tuning both{2, 7, 148, 296}, one{8, 16, 0, 0};
+        mhd_batch_tuning best{}, got{};
+        if (kind == 1) CHECK(mhd_batch_tune(b, 1, &best) == MHD_OK);
+        if (kind >= 2) CHECK(mhd_batch_set_tuning(b, kind == 2 ? &both : &one) == MHD_OK);
+        auto run = [](mhd_batch* x) {
+            mhd_run_info info[2];
+            launches.clear();
+            CHECK(mhd_batch_run(x, 1, info) == MHD_OK);
+            return shape_of_launches();
+        };
+        CHECK(mhd_batch_get_tuning(b, &got) == MHD_OK);
+        if (kind == 1) CHECK(std::memcmp(&got, &best, sizeof got) == 0);
+        run(b);
+        const std::vector<int> was = run(b);
+        CHECK(mhd_batch_set_tuning(b, &got) == MHD_OK && mhd_batch_set_tuning(other, &got) == MHD_OK);
+        run(b);  // captures the graph anew
+        run(other);
+        CHECK(run(b) == was && run(other) == was);
+        CHECK(mhd_batch_destroy(b) == MHD_OK && mhd_batch_destroy(other) == MHD_OK);
+    }
+}
+
 int main() {
+    round_trip();
     no_memory();
     large();
     std::printf("%d failures\n", failures);
