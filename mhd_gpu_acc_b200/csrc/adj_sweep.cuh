@@ -183,7 +183,8 @@ __global__ void __launch_bounds__(32 * AWARPS, AdjShape<R, SOLVER>::kYBlocks)
     R* const sL = sU + NV * 32 * APITCH;                   // [9][32][APITCH], then the results
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ng = U.ng, lo = ng, hi = ng + U.ny;
-    const int i0 = ng + blockIdx.x * AWARPS, j0 = ng - 2 + blockIdx.y * AT - 3;
+    const unsigned across = (U.nx + AWARPS - 1) / AWARPS;  // blocks side by side (one-dimensional launch: any number of rows)
+    const int i0 = ng + blockIdx.x % across * AWARPS, j0 = ng - 2 + blockIdx.x / across * AT - 3;
     double sf = 0.0;
     // thread t: column t % 8, rows t / 8 (all fields of a cell by one thread)
     {
@@ -251,7 +252,7 @@ cudaError_t launch_one(const AdjSweepArgs& a, cudaStream_t st) {
     } else {
         constexpr int bytes = 2 * NV * 32 * APITCH * (int)sizeof(R);
         static_assert(bytes <= 48 * 1024, "the y block's stage needs an opt-in");
-        const dim3 grid((a.U.nx + AWARPS - 1) / AWARPS, (a.U.ny + 4 + AT - 1) / AT);
+        const unsigned grid = (a.U.nx + AWARPS - 1) / AWARPS * ((a.U.ny + 4 + AT - 1) / AT);
         adj_y_kernel<R, LIM, SOLVER><<<grid, 32 * AWARPS, bytes, st>>>(a.U, a.lamOut, a.lamIn, a.Unext, g, gm1, igm1,
                                                                       (R)a.dtd, (R)a.ch, a.damp, a.acc);
     }

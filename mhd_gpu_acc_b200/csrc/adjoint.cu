@@ -125,12 +125,14 @@ __global__ void __launch_bounds__(32) step_scalars_kernel(const double* sc, cons
 // doubled angles give the eight modes) instead of eight sines, and a CTA adds
 // its 16 sums once: 127 -> 14 us at 512^2 FP32.
 constexpr int IC_ROWS = 8;
+__host__ __device__ inline unsigned ic_blocks_across(const DevGrid& g) { return (g.tnx() + 255) / 256; }
 template <typename R>
 __global__ void __launch_bounds__(256) ic_grad_kernel(DevGrid lam, DevGrid U0, double x0, double y0, double dx,
                                                       double dy, double* grad) {
     __shared__ double part[16][8];
     const double T = 2.0 * 3.14159265358979323846, h2 = 0.70710678118654752440, h5 = 0.44721359549995793928;
-    const int i = blockIdx.x * 256 + threadIdx.x, j0 = blockIdx.y * IC_ROWS;
+    const unsigned across = ic_blocks_across(lam);
+    const int i = blockIdx.x % across * 256 + threadIdx.x, j0 = blockIdx.x / across * IC_ROWS;
     double gk[16];
 #pragma unroll
     for (int k = 0; k < 16; ++k) gk[k] = 0.0;
@@ -388,7 +390,8 @@ int gradient(mhd_adjoint* a, const double* amp, double* J, double* grad) {
         }
     }
     // lam_next now holds dJ/dU^0 (ghosts included) and seg[0] U^0: contract with dU^0/da
-    const dim3 grid((a->nx + 4 + 255) / 256, (a->ny + 4 + mhd::adj::IC_ROWS - 1) / mhd::adj::IC_ROWS);
+    // one dimension: the others of a grid end at 65,535 blocks, 524,280 rows here
+    const unsigned grid = mhd::adj::ic_blocks_across(dg(a->seg[0])) * ((a->ny + 4 + mhd::adj::IC_ROWS - 1) / mhd::adj::IC_ROWS);
     if (f64(a))
         mhd::adj::ic_grad_kernel<double><<<grid, 256, 0, st>>>(dg(*lam_next), dg(a->seg[0]), 0.0, 0.0, 1.0 / a->nx, 1.0 / a->ny, a->d_grad);
     else
