@@ -20,9 +20,10 @@
 // with h = 1 / (2 sqrt(x)).  tests/exact_div_check.cu compares both with the
 // operators on random operands and on the hardest roundings.
 //
-// Ranges: |b| in [2^-480, 2^60), numerators +0 or in [2^-960, 2^900) by magnitude,
-// roots of +0 or [2^-900, 2^900): then no quotient, residual or intermediate
-// is subnormal or overflows.
+// Ranges: |b| in [2^-480, 2^60), numerators zero or in [2^-960, 2^540) by magnitude,
+// roots of +0 or [2^-900, 2^900): then quotients lie in (2^-1021, 2^1021), so that none
+// is subnormal or overflows, and the residuals, multiples of 2^-1064, are exact.
+// tests/exact_range_check.cu draws both operands from all of these ranges.
 #pragma once
 
 #include <cmath>
@@ -65,7 +66,7 @@ XD_HD bool xd_out(double a) {
     return (h + h) - lo >= span;
 }
 XD_HD bool out_den(double b) { return xd_out<-480, 60>(b) | (lo_word(b) == 0xffffffffu); }
-XD_HD bool out_num(double a) { return (a != 0.0) & xd_out<-960, 900>(a); }
+XD_HD bool out_num(double a) { return (a != 0.0) & xd_out<-960, 540>(a); }
 // -0, negative and NaN radicands are out of range too (the unsigned difference)
 XD_HD bool out_rad(double x) {
     constexpr unsigned lo = (unsigned)(1023 - 900) << 20, span = 1800u << 20;

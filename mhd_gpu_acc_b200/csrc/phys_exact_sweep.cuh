@@ -441,7 +441,7 @@ MHD_HD_INLINE void slopes(const double* Wm, const double* Wc, const double* Wp, 
         const double n = 2.0 * a * b, d = a + b;  // a b > 0: n > 0 and d has the slopes' sign
         const Recip r = recip(d);
         s[k] = flat ? 0.0 : quot_pos(n, r);
-        bad = bad | (!flat & (out_den(d) | xd_out<-960, 900>(n)));
+        bad = bad | (!flat & (out_den(d) | xd_out<-960, 540>(n)));
     }
     if (bad) {
 #pragma unroll
