@@ -3,7 +3,6 @@
 Per-file flags matter for numerics:
   step_f64.cu   --fmad=false      FP64 step, bit-exact with the reference CPU path
   step_f32.cu   --use_fast_math   FP32-bulk step
-  adj_f32.cu    --use_fast_math   FP32 adjoint sweeps
 Everything else uses the defaults.  The CUDA runtime is linked statically so the
 library only needs the driver at run time.
 
@@ -40,7 +39,7 @@ CU_SOURCES = {
     "batch_api.cu": [],
     "adjoint.cu": [],
     "adj_f64.cu": [],
-    "adj_f32.cu": ["--use_fast_math"],
+    "adj_f32.cu": [],
 }
 CXX_SOURCES = {"cases.cpp": []}
 HEADERS = [f for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))] if os.path.isdir(CSRC) else []

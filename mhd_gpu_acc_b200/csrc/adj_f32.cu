@@ -1,5 +1,4 @@
-// adj_f32.cu -- the FP32 adjoint sweeps.  Build with --use_fast_math, as the
-// FP32-bulk step whose branches they follow (step_f32.cu).
+// adj_f32.cu -- the FP32 adjoint sweeps.
 #include "adj_sweep.cuh"
 
 namespace mhd {

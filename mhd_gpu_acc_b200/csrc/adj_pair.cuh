@@ -54,15 +54,6 @@ ADJ_HD Pr<double> nmad(const Pr<double>& a, const Pr<double>& b, const Pr<double
 template <typename R>
 ADJ_HD Pr<R> operator*(R a, const Pr<R>& b) { return dup(a) * b; }
 
-// Correctly rounded, whatever the translation unit's flags.
-ADJ_HD float rcp_rn(float a) {
-#ifdef __CUDA_ARCH__
-    return __frcp_rn(a);
-#else
-    return 1.0f / a;
-#endif
-}
-ADJ_HD double rcp_rn(double a) { return 1.0 / a; }
 template <typename R>
 ADJ_HD Pr<R> rcp(const Pr<R>& a) { return {rcp(a.x), rcp(a.y)}; }
 
@@ -286,18 +277,10 @@ ADJ_HD void recon_adj2(const R* Wm, const R* Wc, const R* Wp, const Recon<R>& rc
 }
 
 // sqrt(x) and 1 / sqrt(x) for x > 0 (0 and 0 otherwise)
-ADJ_HD void root(float x, float& s, float& is) {
-#ifdef __CUDA_ARCH__
-    is = x > 0.0f ? rsqrtf(x) : 0.0f;
-    s = x * is;
-#else
-    s = x > 0.0f ? std::sqrt(x) : 0.0f;
-    is = x > 0.0f ? 1.0f / s : 0.0f;
-#endif
-}
-ADJ_HD void root(double x, double& s, double& is) {
-    s = x > 0.0 ? sqrt_of(x) : 0.0;
-    is = x > 0.0 ? rcp(s) : 0.0;
+template <typename R>
+ADJ_HD void root(R x, R& s, R& is) {
+    s = x > R(0) ? sqrt(x) : R(0);
+    is = x > R(0) ? rcp(s) : R(0);
 }
 
 // HLL flux of a face and its reverse at once.  U, W, ir: both sides (x = left);

@@ -50,7 +50,7 @@ __device__ __forceinline__ void adj_cell(const R* Uc, const R* lT, int p, int lo
     // c2p with the correctly rounded reciprocal in either precision: the slopes'
     // signs, which a last bit of W can flip where they are at rounding, then do
     // not depend on the build's flags (FP32 gradients moved by 1e-5 otherwise)
-    const R ir = rcp_rn(Uc[RHO]);
+    const R ir = rcp(Uc[RHO]);
     R W[NV];
     c2p_ir(Uc, ir, g, W);
     R Wm[NV], Wp[NV];
