@@ -129,7 +129,7 @@ struct mhd_workspace {
     };
     Device* d = nullptr;
     Host own{};
-    Host* h = nullptr;            // a page-locked slot once something was read back, or &own where there is none
+    Host* h = nullptr;            // a page-locked slot (HostSlots) in place of `own`, or null
     unsigned h_block = 0;         // the block that the slot is of
     void* d_stage = nullptr;      // FP64 staging for uploads/downloads
     size_t stage_bytes = 0;
@@ -144,22 +144,25 @@ struct mhd_workspace {
 
 namespace {
 
-// Page-locked slots for what the device hands back.  Page-locking costs 2 to 4 ms
-// with its release, a hundred times what it saves on a drop-in step, so one block
-// of a fixed size is made when the process first reads something back, shared by
-// its workspaces and kept until the library is unloaded; a workspace returns its
-// slot when it is destroyed.  With every slot taken (or no block to be had) a
-// workspace reads back through its own pageable memory.
-// Measured: create + destroy 4.6 -> 0.75 ms (with a block per workspace before), the
-// CFL maximum of 1000 x 500 cells FP64 22 us with either.
+// Page-locked slots for what the device hands back: the CFL maximum's kernel writes
+// its result there and no copy is queued, which saves 7 us of 30 (1000 x 500 cells FP64).
+// Page-locking costs 2 to 4 ms with its release, some 400 read-backs' worth, so one
+// block of a fixed size is made when the process reads back its kPatience-th maximum
+// (a step loop then, that goes on), shared by its workspaces and kept until the
+// library is unloaded; a workspace returns its slot when it is destroyed.  Without
+// a slot (before that, with every one taken, or with no block to be had) a workspace
+// reads back through its own pageable memory.
+// Measured: create + destroy 4.6 -> 0.75 ms (with a block per workspace before).
 class HostSlots {
     static constexpr size_t kSlot = 128, kSlots = 512;
+    static constexpr int kPatience = 32;
     static_assert(sizeof(mhd_workspace::Host) <= kSlot, "a slot holds a workspace's Host");
     std::mutex lock_;
     char* block_ = nullptr;
     unsigned number_ = 0;  // of the block
     pid_t owner_ = 0;      // a forked child holds no CUDA context
     std::vector<unsigned short> free_;
+    int asked_ = 0;
 
 public:
     mhd_workspace::Host* take(unsigned& block) try {
@@ -170,6 +173,8 @@ public:
             cudaGetLastError();
         }
         if (!block_) {
+            if (++asked_ < kPatience) return nullptr;
+            asked_ = 0;
             std::vector<unsigned short> all(kSlots);
             void* p = nullptr;
             if (cudaHostAlloc(&p, kSlot * kSlots, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
@@ -202,11 +207,7 @@ public:
 };
 HostSlots g_slots;
 
-mhd_workspace::Host* host(mhd_workspace* ws) {
-    if (!ws->h) ws->h = g_slots.take(ws->h_block);
-    if (!ws->h) ws->h = &ws->own;
-    return ws->h;
-}
+mhd_workspace::Host* host(mhd_workspace* ws) { return ws->h ? ws->h : &ws->own; }
 
 // A fault word read back: a bounded device wait that gave up turns into
 // MHD_ERR_TIMEOUT (and the word is cleared).
@@ -221,10 +222,10 @@ int check_fault(mhd_workspace* ws, const char* what) {
     if (cudaMemcpyAsync(&host(ws)->fault, &ws->d->fault, sizeof(int), cudaMemcpyDeviceToHost, ws->stream) != cudaSuccess ||
         cudaStreamSynchronize(ws->stream) != cudaSuccess)
         return fail(MHD_ERR_CUDA, "%s: %s", what, cudaGetErrorString(cudaGetLastError()));
-    return fault_code(ws, ws->h->fault, what);
+    return fault_code(ws, host(ws)->fault, what);
 }
 
-// The clock and the fault word into ws->h, in one copy, after the stream has drained.
+// The clock and the fault word to the host, in one copy, after the stream has drained.
 int read_clock(mhd_workspace* ws) {
     CK(cudaMemcpyAsync(host(ws), ws->d, offsetof(mhd_workspace::Device, fault) + sizeof(int), cudaMemcpyDeviceToHost, ws->stream));
     CK(cudaStreamSynchronize(ws->stream));
@@ -292,8 +293,9 @@ cudaError_t launch_max(const mhd_workspace* ws, const mhd_grid* g, unsigned long
 
 // CFL maximum of g on the host.
 int max_on_host(mhd_workspace* ws, const mhd_grid* g, const char* what, double* mx) {
+    if (!ws->h) ws->h = g_slots.take(ws->h_block);
     mhd_workspace::Host* h = host(ws);
-    const bool pageable = h == &ws->own;
+    const bool pageable = ws->h == nullptr;
     CK(launch_max(ws, g, pageable ? ws->d->max_out : h->max));
     if (pageable) CK(cudaMemcpyAsync(h->max, ws->d->max_out, sizeof h->max, cudaMemcpyDeviceToHost, ws->stream));
     CK(cudaStreamSynchronize(ws->stream));
@@ -500,7 +502,7 @@ int mhd_workspace_destroy(mhd_workspace* ws) {
     if (ws->graph) cudaGraphExecDestroy(ws->graph);
     if (ws->d) cudaFree(ws->d);  // waits for the device
     if (ws->d_stage) cudaFree(ws->d_stage);
-    if (ws->h && ws->h != &ws->own) g_slots.give(ws->h, ws->h_block);
+    if (ws->h) g_slots.give(ws->h, ws->h_block);
     delete ws;
     return MHD_OK;
 }
@@ -771,7 +773,7 @@ int mhd_clock_read(mhd_workspace* ws, mhd_run_info* info) {
     if (!ws || !ws->d) return fail(MHD_ERR_STATE, "mhd_clock_read: null workspace");
     const int crc = read_clock(ws);
     if (crc) return crc;
-    const mhd::DevClock& hc = ws->h->clock;
+    const mhd::DevClock& hc = host(ws)->clock;
     if (hc.steps > 0) ws->ch = hc.last_ch;
     if (info) {
         info->t = hc.t[hc.steps & 1];
@@ -782,7 +784,7 @@ int mhd_clock_read(mhd_workspace* ws, mhd_run_info* info) {
         info->fallbacks = hc.flux_fallbacks;
         info->pad_ = 0;
     }
-    return fault_code(ws, ws->h->fault, "mhd_clock_read");
+    return fault_code(ws, host(ws)->fault, "mhd_clock_read");
 }
 
 int mhd_profile_sweeps(mhd_workspace* ws, mhd_grid* U, mhd_grid* T, double cfl, double t_end, int solver,
@@ -897,7 +899,7 @@ int mhd_run(mhd_workspace* ws, mhd_grid* U, mhd_grid* T, double cfl, double t_en
         info->fallbacks = hc.flux_fallbacks;
         info->pad_ = 0;
     }
-    const int frc = fault_code(ws, ws->h->fault, "mhd_run");
+    const int frc = fault_code(ws, host(ws)->fault, "mhd_run");
     if (frc) return frc;
     const int code = status_code(hc.status);
     if (code != MHD_OK) return fail(code, "mhd_run: step loop stopped with status %d after %d steps", hc.status, hc.steps);

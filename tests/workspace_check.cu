@@ -2,8 +2,8 @@
 // (fake_cuda.h; built and run by test_workspace.py, no GPU).
 //   order: the CFL maximum's accumulator and arrival counter are zero before its
 //   first launch, on a non-blocking stream, with work queued on the default stream.
-//   slots: workspaces share one page-locked block, made at the first read-back and
-//   never by a workspace that reads nothing; each gets its own result from several
+//   slots: workspaces share one page-locked block, made after many read-backs of the
+//   process and never by workspaces that read nothing; each gets its own result from several
 //   threads at once, with more workspaces than slots, and with no block to be had.
 #include <cstdio>
 #include <thread>
@@ -91,8 +91,10 @@ static void slots() {
         mhd_workspace* ws = nullptr;
         CHECK(mhd_workspace_create(&g, &ws) == MHD_OK && mhd_workspace_destroy(ws) == MHD_OK);
     }
+    read_back(3, 2.0);
     CHECK(fake::host_allocs == 0);
-    for (int k = 0; k < 50; ++k) read_back(2, 2.0);
+    for (int k = 0; k < 100; ++k) read_back(2, 2.0);
+    CHECK(fake::host_allocs == 1);
     read_back(700, 2.0);
     std::vector<std::thread> threads;
     for (int t = 0; t < 8; ++t)
@@ -109,7 +111,7 @@ static void slots() {
     std::free(fake::host.begin()->first);
     fake::host.clear();
     for (auto& w : after) CHECK(mhd_workspace_create(&g, &w) == MHD_OK);
-    CHECK(mhd_max_speed(after[0], &g, &v) == MHD_OK);
+    for (int k = 0; k < 300; ++k) CHECK(mhd_max_speed(after[0], &g, &v) == MHD_OK);
     CHECK(mhd_workspace_destroy(before) == MHD_OK);
     CHECK(mhd_max_speed(after[1], &g, &v) == MHD_OK);
     CHECK(fake::host_allocs == 2 && fake::host.size() == 1);
