@@ -3,7 +3,9 @@
 Per-file flags matter for numerics:
   step_f64.cu   --fmad=false      FP64 step, bit-exact with the reference CPU path
   step_f32.cu   --use_fast_math   FP32-bulk step
-Everything else uses the defaults.  The CUDA runtime is linked statically so the
+Everything else uses the defaults.  Device code is not compressed: the FP64 step's
+otherwise would be (from some 10 MB on), and unpacking it cost the first call of a
+process 10 ms (16 -> 6.5 ms).  The CUDA runtime is linked statically so the
 library only needs the driver at run time.
 
 Usage: python -m mhd_gpu_acc_b200.build [--force] [-j N]
@@ -25,7 +27,7 @@ LIB = os.path.join(PKG, "libmhd_b200.so")
 DRIVER = os.path.join(PKG, "mhd_run_case")  # the init / step / output driver (csrc/driver.cpp)
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-NVCC_COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off",
+NVCC_COMMON = ["-std=c++17", "-O3", "-lineinfo", "--no-compress", "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off",
                "-I", os.path.join(ROOT, "include")] + ARCH
 CU_SOURCES = {
     "step_f64.cu": ["--fmad=false"],
