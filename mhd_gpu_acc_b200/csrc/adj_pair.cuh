@@ -158,14 +158,7 @@ ADJ_HD void c2p_adj2(const Pr<R>* W, const Pr<R>& ir, R gm1, const Pr<R>* lW, Pr
     lU[PSI] = lU[PSI] + lW[PSI];
 }
 
-template <typename R>
-ADJ_HD bool finite9(const R* V) {
-    // x * 0 is 0 for a finite x and NaN otherwise
-    R z = V[0] * R(0);
-#pragma unroll
-    for (int k = 1; k < NV; ++k) z = V[k] * R(0) + z;
-    return z == R(0);
-}
+// x * 0 is 0 for a finite x and NaN otherwise
 template <typename R>
 ADJ_HD void physical2(const Pr<R>* V, bool& okx, bool& oky) {
     Pr<R> z = V[0] * dup(R(0));

@@ -112,7 +112,6 @@ struct mhd_workspace {
     double clk_cfl = 0.0, clk_t_end = 0.0;  // of the clock started by mhd_clock_start
     int clk_started = 0;
     double dx = 0.0, dy = 0.0;     // cell spacing of the step; 0 = from the grid's extent
-    int nsm = 148;
     cudaStream_t stream = nullptr;
     struct Device {               // device scratch, one allocation
         mhd::DevClock clock;
@@ -477,10 +476,6 @@ int mhd_workspace_create(const mhd_grid* g, mhd_workspace** out) {
     ws->ny = g->ny;
     ws->ng = g->ng;
     ws->dtype = g->dtype;
-    int dev_id = 0;
-    cudaGetDevice(&dev_id);
-    cudaDeviceGetAttribute(&ws->nsm, cudaDevAttrMultiProcessorCount, dev_id);
-    if (ws->nsm <= 0) ws->nsm = 148;
     if (cudaMalloc(&ws->d, sizeof(mhd_workspace::Device)) != cudaSuccess) {
         mhd_workspace_destroy(ws);
         return fail(MHD_ERR_NOMEM, "mhd_workspace_create: device scratch");

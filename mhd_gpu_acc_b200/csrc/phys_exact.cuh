@@ -14,6 +14,9 @@
 //
 // The functions are __host__ __device__: the host side of the library uses
 // them for the reference's header-inline API (cons_to_prim, riemann_flux).
+// The GPU's sweeps evaluate phys_exact_sweep.cuh, which forms the same values;
+// is_physical, reconstruct and cell_speed are here as the order it is checked
+// against and have no other caller.
 // States are plain double[9] arrays (field order of mhd_common.cuh); the
 // direction is a template parameter so each sweep gets straight-line code.
 #pragma once

@@ -1,5 +1,5 @@
 // step_f64.cu -- the FP64 ("plain") GLM-MHD step: the reference-faithful
-// physics of phys_exact.cuh driven by the fused sweeps of sweep.cuh.
+// physics of phys_exact_sweep.cuh driven by the fused sweeps of sweep.cuh.
 //
 // Build this translation unit with --fmad=false: together with the reference
 // operand order in phys_exact.cuh, whose values phys_exact_sweep.cuh forms, it

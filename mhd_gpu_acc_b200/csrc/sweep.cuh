@@ -456,10 +456,13 @@ __host__ __device__ inline SweepPlan y_plan(int rows, int per) {
 // but the launch ends on stragglers of one task's length: the sum is least at
 // len ~ sqrt(N), with the factor `c` measured per sweep and precision and `cap`
 // the longest worth taking (the large-grid lengths, kXRpw and kYBand).  Up to
-// `one_wave` iterations per slot the tasks all run at once, and the shortest
-// length that still fits them in one wave is best (x: 4, y: 11; e.g. FP32 y at
-// 512^2, N = 3.7: 53 / 38 / 37 / 31 / 33 / 36 us with 1 / 2 / 3 / 4 / 5 / 6
-// rows; at 768^2, N = 8.1, 41.9 us with 9 rows against 49.0 with 5).  Measured
+// `one_wave` iterations per slot (x: 4, y: 11) equal tasks of ceil(N) iterations
+// are best: one wave of them, or a little more -- in x up to a fifth more tasks than
+// slots, as a segment is four cells short of its chunks (lengthening the segments
+// until one wave holds them measured the same from 128^2 to 512^2 in both precisions:
+// FP32 512^2 20.6 us with 2560 tasks on 2368 slots and with 2048).  E.g. FP32 y at
+// 512^2, N = 3.7: 53 / 38 / 37 / 31 / 33 / 36 us with 1 / 2 / 3 / 4 / 5 / 6 rows; at
+// 768^2, N = 8.1, 41.9 us with 9 rows against 49.0 with 5.  Measured
 // (HLLD, van Leer, us; with the cap's length at every size ->
 // by this rule): FP32 x 512^2 35 -> 22, 1024^2 55 -> 48, y 512^2 107 -> 31,
 // 1024^2 121 -> 72, 2048^2 202 -> 183; FP64 x 512^2 64 -> 55, 1024^2 173 -> 160,
