@@ -471,8 +471,8 @@ def run_ours(a, world, rank, local):
 
 
 def run_batch(a, world, rank, local):
-    """256 Orszag-Tang instances of uneven size (sides U{64..1024}), one persistent
-    launch per sweep phase, autotuned.  With N ranks the one batch is split over
+    """256 Orszag-Tang instances of uneven size (sides U{64..1024}), one launch per
+    sweep phase, autotuned.  With N ranks the one batch is split over
     the GPUs by LPT on cells (strong scaling, no data-path collective); the time
     is the max over ranks and the value all ranks' cell-updates over it."""
     import numpy as np

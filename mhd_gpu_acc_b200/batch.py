@@ -1,5 +1,5 @@
 """Batched instances: many independent MHD problems of uneven size advanced by
-one persistent launch per sweep phase and a CUDA-graph step loop (mhd_batch_*
+one launch per sweep phase and a CUDA-graph step loop (mhd_batch_*
 in include/mhd_b200.h)."""
 from __future__ import annotations
 

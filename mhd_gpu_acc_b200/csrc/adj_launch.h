@@ -26,10 +26,12 @@ cudaError_t launch_adj_sweep_f64(const AdjSweepArgs& a, cudaStream_t st);
 cudaError_t launch_adj_sweep_f32(const AdjSweepArgs& a, cudaStream_t st);
 
 // Resident CTAs that the register budgets are cut for: y CTAs of 8 warps, x CTAs
-// of 4.  Measured per sweep: FP32 HLL at 512^2 y 37 us with 2 (128 registers, 0.4
-// KB of spills) against 42 us with 1 (237, none); x 29.6 us with 3 x 4 warps (168)
-// against 30.5 us with 2 x 8 (128) and 36 us with 1 x 8 (235); FP64 HLLD at 256^2 x
-// 48.5 us with 2 x 4 against 50.3 us with 1 x 8 (255 either way).
+// of 4.  Measured per sweep: FP32 HLL at 512^2 y 37 us with 2 (128 registers, 0.2
+// KB of spills) against 42 us with 1 (237, none); x 30 us with 3 x 4 warps (168);
+// FP32 HLLD y 74, x 56 us; FP64 at 256^2 HLL y 29, x 21 us, HLLD y 57, x 52 us.  Shapes
+// compared with reciprocals good to 2 ulp (FP32: fast math): FP32 HLL x 29.6 us
+// against 30.5 us with 2 x 8 warps (128) and 36 us with 1 x 8 (235); FP64 HLLD x 48.5 us
+// with 2 x 4 against 50.3 us with 1 x 8 (255 either way).
 template <typename R, int SOLVER>
 struct AdjShape;
 template <int SOLVER>

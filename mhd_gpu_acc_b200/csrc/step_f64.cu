@@ -24,9 +24,10 @@ struct ExactPolicy {
     // The face-side states carry their primitives and 1 / rho, and quotients and
     // roots come in branch-free groups (phys_exact_sweep.cuh): at 4096^2 (HLLD, van
     // Leer) x 2.044 -> 1.440 ms, y 2.373 -> 1.690 ms, at 2048^2 x 0.591 -> 0.395,
-    // y 0.687 -> 0.492 ms, bit-identical results (x 1.348, y 1.586 ms since the
-    // one-offset cell addresses and the four-value positivity tests).  They wait on FP64
-    // latency (2 warps per scheduler, FP64 pipe 50 % busy, 37 % before).
+    // y 0.687 -> 0.492 ms, bit-identical results (4096^2 x 1.34, y 1.63 ms, 2048^2 x
+    // 0.368, y 0.468 ms since the one-offset cell addresses and the four-value
+    // positivity tests).  They wait on FP64 latency (2 warps per scheduler, FP64 pipe
+    // 55 % busy in x and 51 % in y, 37 % before).
     // y-sweep window in shared memory (y_segment_carried), 2 CTAs per SM.
     // Measured before that at 4096^2 (HLLD, van Leer): 2.97 ms, against 3.11 ms for the
     // register window (255 registers, spills) and 3.06 ms for the shared-memory
