@@ -127,6 +127,7 @@ struct mhd_workspace {
         unsigned long long max[2];  // CFL maximum bits, fault word
     };
     Device* d = nullptr;
+    cudaEvent_t cleared = nullptr;  // the scratch is zero
     Host own{};
     Host* h = nullptr;            // a page-locked slot (HostSlots) in place of `own`, or null
     unsigned h_block = 0;         // the block that the slot is of
@@ -480,10 +481,9 @@ int mhd_workspace_create(const mhd_grid* g, mhd_workspace** out) {
         mhd_workspace_destroy(ws);
         return fail(MHD_ERR_NOMEM, "mhd_workspace_create: device scratch");
     }
-    // zero before any launch on whatever stream the workspace is given (a
-    // non-blocking one does not wait for the default stream)
     cudaError_t e = cudaMemsetAsync(ws->d, 0, offsetof(mhd_workspace::Device, diag), nullptr);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ws->cleared, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventRecord(ws->cleared, nullptr);
     if (e != cudaSuccess) {
         mhd_workspace_destroy(ws);
         return fail(MHD_ERR_CUDA, "mhd_workspace_create: %s", cudaGetErrorString(e));
@@ -496,6 +496,7 @@ int mhd_workspace_destroy(mhd_workspace* ws) {
     if (!ws) return MHD_OK;
     if (ws->graph) cudaGraphExecDestroy(ws->graph);
     if (ws->d) cudaFree(ws->d);  // waits for the device
+    if (ws->cleared) cudaEventDestroy(ws->cleared);
     if (ws->d_stage) cudaFree(ws->d_stage);
     if (ws->h) g_slots.give(ws->h, ws->h_block);
     delete ws;
@@ -504,11 +505,25 @@ int mhd_workspace_destroy(mhd_workspace* ws) {
 
 int mhd_workspace_set_stream(mhd_workspace* ws, void* stream) {
     if (!ws) return fail(MHD_ERR_STATE, "mhd_workspace_set_stream: null workspace");
-    if (ws->stream != static_cast<cudaStream_t>(stream) && ws->graph) {
+    const cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (ws->stream != st && ws->graph) {
         cudaGraphExecDestroy(ws->graph);
         ws->graph = nullptr;
     }
-    ws->stream = static_cast<cudaStream_t>(stream);
+    // A non-blocking stream does not wait for the default stream, where the scratch
+    // was cleared (on the GPU only, so that the host need not wait for what is
+    // queued there); a stream in capture cannot wait for an event from outside.
+    if (st != nullptr) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        const cudaError_t e = cudaStreamIsCapturing(st, &capture);
+        if (e == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+            CK(cudaStreamWaitEvent(st, ws->cleared, 0));
+        } else {
+            cudaGetLastError();
+            CK(cudaEventSynchronize(ws->cleared));
+        }
+    }
+    ws->stream = st;
     return MHD_OK;
 }
 

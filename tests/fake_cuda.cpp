@@ -34,7 +34,10 @@ cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind k) {
     return cudaSuccess;
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t st) {
-    if (st == nullptr) fake::drain();
+    if (st == nullptr) {
+        ++fake::default_waits;
+        fake::drain();
+    }
     return cudaSuccess;
 }
 cudaError_t cudaDeviceSynchronize() {
@@ -56,10 +59,20 @@ cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) {
     if (fake::graph_launch) fake::graph_launch();
     return cudaSuccess;
 }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { *e = (cudaEvent_t)8; return cudaSuccess; }
+cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* s) { *s = fake::capturing; return cudaSuccess; }
+// events are recorded on the default stream only
+cudaError_t cudaStreamWaitEvent(cudaStream_t st, cudaEvent_t, unsigned) {
+    if (st != nullptr) fake::drain();
+    return fake::capturing == cudaStreamCaptureStatusNone ? cudaSuccess : cudaErrorStreamCaptureIsolation;
+}
 cudaError_t cudaEventCreate(cudaEvent_t* e) { *e = (cudaEvent_t)8; return cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t) {
+    fake::drain();
+    return cudaSuccess;
+}
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 1.0f; return cudaSuccess; }
 void** __cudaRegisterFatBinary(void*) { static void* h; return &h; }
 void __cudaRegisterFatBinaryEnd(void**) {}

@@ -21,6 +21,8 @@ inline std::vector<std::function<void()>> queued;  // on the default stream
 inline std::map<char*, size_t> device, host;       // live allocations
 inline int mallocs = 0, host_allocs = 0, fail_malloc_at = -1;
 inline bool fail_host = false;
+inline int default_waits = 0;  // of the host for the default stream
+inline cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;  // of every stream asked about
 inline std::function<void()> graph_launch;  // what a launch of the captured graph does
 inline bool hollow = false;  // device blocks over 1 GB get a page only (their contents are not looked at)
 

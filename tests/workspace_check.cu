@@ -1,7 +1,8 @@
 // Host-side checks of the workspace's scratch (csrc/capi.cu) on a fake runtime
 // (fake_cuda.h; built and run by test_workspace.py, no GPU).
 //   order: the CFL maximum's accumulator and arrival counter are zero before its
-//   first launch, on a non-blocking stream, with work queued on the default stream.
+//   first launch, on a non-blocking stream, with work queued on the default stream,
+//   for which the host does not wait.
 //   slots: workspaces share one page-locked block, made after many read-backs of the
 //   process and never by workspaces that read nothing; each gets its own result from several
 //   threads at once, with more workspaces than slots, and with no block to be had.
@@ -50,13 +51,18 @@ static mhd_grid shape() {
 
 static void order() {
     const mhd_grid g = shape();
-    mhd_workspace* ws = nullptr;
-    CHECK(mhd_workspace_create(&g, &ws) == MHD_OK);
-    CHECK(mhd_workspace_set_stream(ws, (void*)16) == MHD_OK);
-    double dt = 0.0;
-    CHECK(mhd_set_gamma(ws, 2.0) == MHD_OK);
-    CHECK(mhd_compute_dt(ws, &g, 0.4, &dt) == MHD_OK && dt == 0.4 / 16 / 2.0);
-    CHECK(mhd_workspace_destroy(ws) == MHD_OK);
+    for (const bool capture : {false, true}) {
+        mhd_workspace* ws = nullptr;
+        const int waits = fake::default_waits;
+        CHECK(mhd_workspace_create(&g, &ws) == MHD_OK && fake::default_waits == waits);
+        fake::capturing = capture ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
+        CHECK(mhd_workspace_set_stream(ws, (void*)16) == MHD_OK);
+        fake::capturing = cudaStreamCaptureStatusNone;
+        double dt = 0.0;
+        CHECK(mhd_set_gamma(ws, 2.0) == MHD_OK);
+        CHECK(mhd_compute_dt(ws, &g, 0.4, &dt) == MHD_OK && dt == 0.4 / 16 / 2.0);
+        CHECK(mhd_workspace_destroy(ws) == MHD_OK);
+    }
     CHECK(fake::device.empty());
 }
 
