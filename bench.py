@@ -606,7 +606,7 @@ def run_adjoint(a, world, rank, local):
             "value": out["fp32"]["gradient_over_forward"], "unit": "x forward", "n_gpus": 1, "steps": steps,
             "higher_is_better": False, "dtype": "f32",
             "config": {"workload": f"orszag_tang_adjoint_{n}x{n}_{steps}steps_hll_vanleer", "seed": a.seed,
-                       "checkpoints": "every ~sqrt(N) steps"},
+                       "checkpoints": "all steps stored where memory has room, else every ~sqrt(N)"},
             "fp32": {k: v for k, v in out["fp32"].items() if k != "grad"},
             "fp64": {k: v for k, v in out["fp64"].items() if k != "grad"},
             "fp32_vs_fp64_grad_rel": float(np.linalg.norm(g32 - g64) / np.linalg.norm(g64)),
